@@ -5,8 +5,10 @@
 #include <cctype>
 #include <chrono>
 #include <climits>
+#include <cmath>
 #include <cstring>
 #include <memory>
+#include <numeric>
 #include <string>
 
 #include "../../include/gat.h"
@@ -1317,7 +1319,7 @@ struct gat_batch {
     gat_config cfg{};
     bool prepared = false, use_graph = false;
     int tile = 32, block = 256, grid = 0, chunk = 8;
-    int64_t vtotal = 0, stride = 0;
+    int64_t vtotal = 0, units = 0, stride = 0;  // queue grabs, level-1 units
     GatPlan *d_plans = nullptr;
     void *d_jobs = nullptr;
     int64_t *d_vstart = nullptr;
@@ -1418,13 +1420,30 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
     std::vector<unsigned char> host_jobs(J * jb);
     std::vector<GatPlan> plans(J);
     std::vector<int64_t> vstart(J);
+    // The queue's order: plans with more levels first, and of those the jobs
+    // with the longest rows, so that a job of heavy units does not start when
+    // the others are nearly done.
+    std::vector<size_t> order(J);
+    std::iota(order.begin(), order.end(), size_t(0));
+    auto weight = [&](size_t j) {
+        const GatPlan &p = b->jobs[j].s->plan.plan;
+        return std::make_pair(p.basic, double(b->jobs[j].g->host.E) *
+                                           std::pow(double(b->jobs[j].g->host.max_degree()),
+                                                    double(p.basic - 1)));
+    };
+    std::vector<std::pair<int32_t, double>> weights(J);
+    for (size_t j = 0; j < J; j++) weights[j] = weight(j);
+    std::stable_sort(order.begin(), order.end(),
+                     [&](size_t x, size_t y) { return weights[x] > weights[y]; });
     b->divisors.assign(J, 1);
     b->modes.assign(J, 0);
     cudaError_t e;
     if ((e = cudaMalloc(&b->d_plans, sizeof(GatPlan) * J)) != cudaSuccess)
         return fail(GAT_ERR_MEMORY, "batch plans");
-    int64_t stride = 0, vt = 0;
-    for (size_t j = 0; j < J; j++) {
+    int64_t stride = 0;
+    b->units = 0;
+    for (size_t q = 0; q < J; q++) {
+        const size_t j = order[q];
         gat_graph *g = b->jobs[j].g;
         const gat_schedule *s = b->jobs[j].s;
         const bool exact = s->mode == GAT_MODE_EXACT;
@@ -1450,17 +1469,14 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
         v.bitmap_words = dc.bitmap_words;
         plans[j] = s->plan.plan;
         if (b->cfg.special_kernels == 0) plans[j].lane_last = 0;
-        batch_fill_job(host_jobs.data() + j * jb, b->d_plans + j, plans[j], v,
-                       b->cfg.set_search_type, b->cfg.hub_bitmaps != 0, b->jobs[j].shard,
-                       b->jobs[j].num_shards);
+        batch_fill_job(host_jobs.data() + q * jb, b->d_plans + j, plans[j], v,
+                       b->cfg.set_search_type, b->cfg.hub_bitmaps != 0, (int)j,
+                       b->jobs[j].shard, b->jobs[j].num_shards);
         stride = std::max<int64_t>(stride, tile_scratch_ints(plans[j], v.max_degree));
-        vstart[j] = vt;
-        const int64_t n = batch_job_tasks(host_jobs.data() + j * jb);
-        vt += (n + b->chunk - 1) / b->chunk * b->chunk;
+        b->units += batch_job_tasks(host_jobs.data() + q * jb);
         b->divisors[j] = plans[j].divisor;
         b->modes[j] = s->mode;
     }
-    b->vtotal = vt;
     b->stride = stride;
     int occ = batch_blocks_per_sm(b->tile, b->block);
     if (occ <= 0) return fail(GAT_ERR_CUDA, "batch kernel does not fit on the device");
@@ -1473,6 +1489,12 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
     if (per_block > 0) {
         if (per_block > budget) return fail(GAT_ERR_MEMORY, "memory budget below one CTA's scratch");
         b->grid = (int)std::min<int64_t>(b->grid, budget / per_block);
+    }
+    b->vtotal = 0;
+    for (size_t q = 0; q < J; q++) {
+        vstart[q] = b->vtotal;
+        b->vtotal += batch_job_grabs(host_jobs.data() + q * jb, plans[order[q]],
+                                     int64_t(b->grid) * (b->block / b->tile), b->tile, b->chunk);
     }
     b->scratch_bytes = size_t(std::max<int64_t>(per_block * b->grid, 4));
     if ((e = cudaMalloc(&b->d_jobs, J * jb)) != cudaSuccess ||
@@ -1498,7 +1520,7 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
         cudaMemsetAsync(b->d_cursor, 0, sizeof(unsigned long long), b->stream);
         cudaMemsetAsync(b->d_results, 0, sizeof(unsigned long long) * J, b->stream);
         cudaError_t le = launch_batch(b->d_jobs, b->d_vstart, (int32_t)J, b->vtotal, b->tile,
-                                      b->grid, b->block, b->chunk, b->d_cursor, b->d_results,
+                                      b->grid, b->block, b->d_cursor, b->d_results,
                                       b->d_scratch, b->stride, b->stream);
         cudaMemcpyAsync(b->h_results, b->d_results, sizeof(unsigned long long) * J,
                         cudaMemcpyDeviceToHost, b->stream);
@@ -1525,7 +1547,7 @@ int gat_batch_run(gat_batch *b, gat_stats *stats) {
         cudaMemsetAsync(b->d_cursor, 0, sizeof(unsigned long long), b->stream);
         cudaMemsetAsync(b->d_results, 0, sizeof(unsigned long long) * J, b->stream);
         e = launch_batch(b->d_jobs, b->d_vstart, (int32_t)J, b->vtotal, b->tile, b->grid,
-                         b->block, b->chunk, b->d_cursor, b->d_results, b->d_scratch, b->stride,
+                         b->block, b->d_cursor, b->d_results, b->d_scratch, b->stride,
                          b->stream);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(b->h_results, b->d_results, sizeof(unsigned long long) * J,
@@ -1554,7 +1576,7 @@ int gat_batch_run(gat_batch *b, gat_stats *stats) {
         st.block = b->block;
         st.tile = b->tile;
         st.launches = 1;
-        st.tasks = (uint64_t)b->vtotal;
+        st.tasks = (uint64_t)b->units;
         st.scratch_bytes = (int64_t)b->scratch_bytes;
         *stats = st;
     }

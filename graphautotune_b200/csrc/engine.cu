@@ -7,8 +7,8 @@
 //
 //  * The level-1 units (v0, v1) are the work queue.  They are numbered by
 //    CSR entry (or, when the plan bounds v1 < v0, by entry among each row's
-//    lower neighbours) and handed out in chunks through one atomic cursor,
-//    which balances power-law rows across the grid.
+//    lower neighbours) and handed out in grabs of at most `chunk` through
+//    one atomic cursor, which balances power-law rows across the grid.
 //  * A tile of G lanes (G = the reference's threads_per_warp knob) owns one
 //    unit at a time and walks levels 2 .. basic-1 depth-first; its state
 //    (embedding, per-level candidate cursor, per-prefix set descriptor) lives
@@ -76,10 +76,12 @@ struct SearchArgs {
 };
 
 // One job of a batched launch: a plan on a graph, over the level-1 units
-// [task_begin, num_tasks) (ctr, scratch and chunk of `args` are unused; the
-// batch supplies them).
+// [task_begin, num_tasks), args.chunk of them per queue grab (ctr and scratch
+// of `args` are unused; the batch supplies them).
 struct BatchJob {
     SearchArgs args;
+    int32_t result;  // where the job's total goes
+    int32_t pad;
 };
 
 template <int G>
@@ -566,170 +568,318 @@ __device__ __forceinline__ int32_t cut_serial(const SearchArgs &a, int32_t v,
     return lower_serial(nb, dv, T);
 }
 
+// What a lane reads of the levels before the one it forms: the tile's state
+// in shared memory (TileState), or, for two-level plans, a root of the
+// lane's own (PairState: every level-0 set is N(v0), cut at v0 when its
+// bound says so).
+struct TileState {
+    const TileSmem &S;
+    __device__ __forceinline__ int32_t v(int j) const { return S.v[j]; }
+    __device__ __forceinline__ const int32_t *set(int f) const { return S.sp[f]; }
+    __device__ __forceinline__ int32_t len(const GatPlan &, int f) const { return S.sl[f]; }
+    __device__ __forceinline__ int32_t owner(int f) const { return S.owner[f]; }
+};
+
+struct PairState {
+    int32_t v0, d0, lo0;
+    const int32_t *nb0;
+    __device__ __forceinline__ int32_t v(int) const { return v0; }
+    __device__ __forceinline__ const int32_t *set(int) const { return nb0; }
+    __device__ __forceinline__ int32_t len(const GatPlan &P, int f) const {
+        return (P.p_trunc[f] & 1u) ? lo0 : d0;
+    }
+    __device__ __forceinline__ int32_t owner(int) const { return v0; }
+};
+
+template <class State>
+__device__ __forceinline__ int32_t min_level(const State &st, unsigned m) {
+    int32_t r = kInf;
+    while (m) {
+        const int j = __ffs(m) - 1;
+        m &= m - 1;
+        r = min(r, st.v(j));
+    }
+    return r;
+}
+
 // y equals one of the levels in `ex` (bit k stands for the lane's candidate).
-__device__ __forceinline__ bool excluded(const TileSmem &S, unsigned ex, int k, int32_t cand,
+template <class State>
+__device__ __forceinline__ bool excluded(const State &st, unsigned ex, int k, int32_t cand,
                                          int32_t y) {
     bool r = ((ex >> k) & 1u) && y == cand;
     unsigned m = ex & ~(1u << k);
     while (m) {
         const int j = __ffs(m) - 1;
         m &= m - 1;
-        r |= (S.v[j] == y);
+        r |= (st.v(j) == y);
     }
     return r;
 }
 
-// Last level with one candidate per lane (plans with lane_last set).  Every
-// set of level k = basic-1 is either a count |N(cand) n F| whose father F
-// belongs to an earlier level or N(cand) itself, so nothing of level k has to
-// be stored: lane i takes candidates i, i+G, ... of the level's loop list and
-// forms that level's sets and the unit's IEP value alone (IEP slots of
-// earlier levels are read from the tile's state).  No shared-memory writes,
-// no syncs, and no idle lanes when the lists are shorter than the tile.  Each
-// set and each IEP value is formed exactly as level_sets and iep_value form
-// it for that candidate (same bounds, exclusions and bitmap-or-search
-// choice).  Returns the sum of the candidates' IEP values on every lane.
-// The candidates are src[i] for i in [i0, i1): the level's loop list (k >= 2),
-// or, at k = 1, the slice of N(v0) that holds the chunk's level-1 units.
+// Candidate `cand` equals an earlier level it must differ from.
+template <class State>
+__device__ __forceinline__ bool collides(const State &st, const GatPlan &P, int k,
+                                         int32_t cand) {
+    bool hit = false;
+    unsigned dm = P.l_distinct[k];
+    while (dm) {
+        const int j = __ffs(dm) - 1;
+        dm &= dm - 1;
+        hit |= (st.v(j) == cand);
+    }
+    return hit;
+}
+
+// List elements one lane would walk for this candidate's sets (the shorter
+// list of each intersection, before bounds).
+template <class State>
+__device__ __forceinline__ int32_t lane_cost(const State &st, const GatPlan &P, int k,
+                                             int32_t dv) {
+    int32_t c = 0;
+    for (int p = P.l_pbegin[k]; p < P.l_pbegin[k + 1]; p++)
+        if (P.p_kind[p] == GAT_SET_COUNT) c += min(dv, st.len(P, P.p_father[p]));
+    return c;
+}
+
+// The IEP value of one last-level candidate (level k = basic-1), formed by
+// one lane alone.  Every set of that level is either a count |N(cand) n F|
+// whose father F belongs to an earlier level or N(cand) itself, so nothing
+// has to be stored.  Each set and each IEP value is formed exactly as
+// level_sets and iep_value form it (same bounds, exclusions and
+// bitmap-or-search choice).  `i` is the candidate's position in its list.
+template <bool STATS, class State>
+__device__ __forceinline__ unsigned long long lane_candidate(const State &st, const GatPlan &P,
+                                                             const SearchArgs &a, int k,
+                                                             int32_t cand, int i, bool hit,
+                                                             unsigned long long &by) {
+    const unsigned kbit = 1u << k;
+    const int loop = P.l_loop[k];
+    const int pb = P.l_pbegin[k], pe = P.l_pbegin[k + 1];
+    long long lv[8];   // level-k sets: count, or cut length of N(cand)
+    long long val[8];  // IEP slots
+    const int64_t o = a.off[cand];
+    const int32_t *nb = a.adj + o;
+    const int32_t dv = (int32_t)(a.off[cand + 1] - o);
+    const int hub_v = (a.hub_slot != nullptr) ? a.hub_slot[cand] : -1;
+    for (int p = pb; p < pe; p++) {
+        if (hit) {
+            lv[p - pb] = 0;
+            continue;
+        }
+        const unsigned tm = P.p_trunc[p];
+        int32_t T = min_level(st, tm & ~kbit);
+        if (tm & kbit) T = min(T, cand);
+        if (P.p_kind[p] == GAT_SET_ALIAS) {
+            lv[p - pb] = cut_serial(a, cand, nb, dv, T);
+            continue;
+        }
+        const int f = P.p_father[p];
+        const int32_t *fp = st.set(f);
+        int32_t fl = st.len(P, f);
+        if (T != kInf) {
+            if (T == cand && f == loop)
+                fl = min(fl, i);
+            else if (tm != P.p_trunc[f])
+                fl = lower_serial(fp, fl, T);
+        }
+        const int owner_f = st.owner(f);
+        const int hub_f = (a.hub_slot != nullptr && owner_f >= 0) ? a.hub_slot[owner_f] : -1;
+        const uint32_t *row = nullptr;
+        const int32_t *probe = nullptr;
+        int np = 0;
+        int32_t nl = dv;
+        if (hub_v >= 0 && fl <= dv) {
+            row = a.bitmaps + (int64_t)hub_v * a.bitmap_words;
+            probe = fp;
+            np = fl;
+            if (STATS) nl = cut_serial(a, cand, nb, dv, T);
+        } else {
+            nl = cut_serial(a, cand, nb, dv, T);
+            const int shorter = min(nl, fl), longer = max(nl, fl);
+            const long long bs_cost = (long long)shorter * ceil_log2(longer + 1);
+            if (hub_v >= 0 && (long long)fl <= bs_cost && (hub_f < 0 || fl <= nl)) {
+                row = a.bitmaps + (int64_t)hub_v * a.bitmap_words;
+                probe = fp;
+                np = fl;
+            } else if (hub_f >= 0 && (long long)nl <= bs_cost) {
+                row = a.bitmaps + (int64_t)hub_f * a.bitmap_words;
+                probe = nb;
+                np = nl;
+            }
+        }
+        if (STATS) by += 4ull * (unsigned)(nl + fl);
+        const unsigned ex = P.p_excl[p];
+        int c = 0;
+        if (row) {
+            for (int e = 0; e < np; e++) {
+                const int32_t y = probe[e];
+                c += (bit_set(row, y) && !excluded(st, ex, k, cand, y)) ? 1 : 0;
+            }
+        } else {
+            const int32_t *sa = nl <= fl ? nb : fp;
+            const int32_t *lb = nl <= fl ? fp : nb;
+            const int ns = min(nl, fl), nlong = max(nl, fl);
+            if (nlong >= a.linear_below && merge_pays(ns, nlong)) {
+                merge_walk(sa, 0, ns, lb, nlong, [&](int32_t y) {
+                    c += excluded(st, ex, k, cand, y) ? 0 : 1;
+                });
+            } else {
+                for (int e = 0; e < ns; e++) {
+                    const int32_t y = sa[e];
+                    c += (contains(lb, nlong, y, a.linear_below) &&
+                          !excluded(st, ex, k, cand, y))
+                             ? 1
+                             : 0;
+                }
+            }
+        }
+        lv[p - pb] = c;
+    }
+    for (int x = 0; x < P.iep_num; x++) {
+        const int p = P.iep_prefix[x];
+        const bool here = P.p_level[p] == k;
+        if (P.p_kind[p] == GAT_SET_COUNT) {
+            val[x] = here ? lv[p - pb] : (long long)st.len(P, p);
+            continue;
+        }
+        const int32_t *ptr = here ? nb : st.set(p);
+        int32_t len = here ? (int32_t)lv[p - pb] : st.len(P, p);
+        const unsigned bm = P.iep_bound[x];
+        int32_t B = min_level(st, bm & ~kbit);
+        if (bm & kbit) B = min(B, cand);
+        if (B != kInf) len = lower_serial(ptr, len, B);
+        const unsigned m = P.iep_sub[x];
+        int h = 0;
+        for (int j = 0; j < P.basic; j++)
+            if ((m >> j) & 1u)
+                h += contains(ptr, len, j == k ? cand : st.v(j), a.linear_below) ? 1 : 0;
+        val[x] = (long long)len - h;
+    }
+    unsigned long long local = 0, cur = 1;
+    int last = -1;
+    for (int g = 0; g < P.num_terms; g++) {
+        const unsigned long long v = (unsigned long long)val[P.t_slot[g]];
+        cur = (g == last + 1) ? v : cur * v;
+        if (P.t_close[g]) {
+            last = g;
+            local += cur * (unsigned long long)(long long)P.t_coef[g];
+        }
+    }
+    return local;
+}
+
+// A lane's candidate is handed to the whole tile when its lists are this
+// much longer than the tile's average: the other lanes would wait for it.
+// The constant is the cost of one cooperative candidate (its shared-memory
+// writes and tile syncs) in list elements.
+constexpr int32_t kHeavyBase = 192;
+constexpr int32_t kHeavyFactor = 4;
+
+template <int G>
+__device__ __forceinline__ unsigned heavy_lanes(const Tile<G> &t, int32_t cost) {
+    if (G < 8) return 0u;
+    const int32_t mean = t.sum(min(cost, 1 << 24)) / G;
+    return t.ballot(cost > kHeavyBase + kHeavyFactor * mean);
+}
+
+// Last level with one candidate per lane (plans with lane_last set): lane i
+// of the tile takes candidates i, i+G, ... of the level's loop list
+// src[0, n) (lane_candidate).  No shared-memory writes, no syncs, and no idle
+// lanes when the lists are shorter than the tile.  Returns the sum of the
+// candidates' IEP values on every lane.
 template <int G, bool STATS>
 __device__ unsigned long long lane_last_level(const Tile<G> &t, const TileSmem &S,
                                               const GatPlan &P, const SearchArgs &a, int k,
                                               unsigned long long &bytes, const int32_t *src,
-                                              int i0, int i1) {
-    const unsigned kbit = 1u << k;
-    const int loop = P.l_loop[k];
-    const int pb = P.l_pbegin[k], pe = P.l_pbegin[k + 1];
+                                              int n) {
+    const TileState st{S};
     unsigned long long sum = 0, by = 0;
-    long long lv[8];   // level-k sets: count, or cut length of N(cand)
-    long long val[8];  // IEP slots
-    for (int i = i0 + t.lane; i < i1; i += G) {
+    for (int i = t.lane; i < n; i += G) {
         const int32_t cand = src[i];
-        bool hit = false;
-        unsigned dm = P.l_distinct[k];
-        while (dm) {
-            const int j = __ffs(dm) - 1;
-            dm &= dm - 1;
-            hit |= (S.v[j] == cand);
-        }
+        const bool hit = collides(st, P, k, cand);
         // Exact plans skip a colliding candidate; reference plans keep it
         // with every level-k set empty.
         if (hit && !P.collide_clear) continue;
-        const int64_t o = a.off[cand];
-        const int32_t *nb = a.adj + o;
-        const int32_t dv = (int32_t)(a.off[cand + 1] - o);
-        const int hub_v = (a.hub_slot != nullptr) ? a.hub_slot[cand] : -1;
-        for (int p = pb; p < pe; p++) {
-            if (hit) {
-                lv[p - pb] = 0;
-                continue;
-            }
-            const unsigned tm = P.p_trunc[p];
-            int32_t T = min_of(S, tm & ~kbit);
-            if (tm & kbit) T = min(T, cand);
-            if (P.p_kind[p] == GAT_SET_ALIAS) {
-                lv[p - pb] = cut_serial(a, cand, nb, dv, T);
-                continue;
-            }
-            const int f = P.p_father[p];
-            const int32_t *fp = S.sp[f];
-            int32_t fl = S.sl[f];
-            if (T != kInf) {
-                if (T == cand && f == loop)
-                    fl = min(fl, i);
-                else if (tm != P.p_trunc[f])
-                    fl = lower_serial(fp, fl, T);
-            }
-            const int owner_f = S.owner[f];
-            const int hub_f =
-                (a.hub_slot != nullptr && owner_f >= 0) ? a.hub_slot[owner_f] : -1;
-            const uint32_t *row = nullptr;
-            const int32_t *probe = nullptr;
-            int np = 0;
-            int32_t nl = dv;
-            if (hub_v >= 0 && fl <= dv) {
-                row = a.bitmaps + (int64_t)hub_v * a.bitmap_words;
-                probe = fp;
-                np = fl;
-                if (STATS) nl = cut_serial(a, cand, nb, dv, T);
-            } else {
-                nl = cut_serial(a, cand, nb, dv, T);
-                const int shorter = min(nl, fl), longer = max(nl, fl);
-                const long long bs_cost = (long long)shorter * ceil_log2(longer + 1);
-                if (hub_v >= 0 && (long long)fl <= bs_cost && (hub_f < 0 || fl <= nl)) {
-                    row = a.bitmaps + (int64_t)hub_v * a.bitmap_words;
-                    probe = fp;
-                    np = fl;
-                } else if (hub_f >= 0 && (long long)nl <= bs_cost) {
-                    row = a.bitmaps + (int64_t)hub_f * a.bitmap_words;
-                    probe = nb;
-                    np = nl;
-                }
-            }
-            if (STATS) by += 4ull * (unsigned)(nl + fl);
-            const unsigned ex = P.p_excl[p];
-            int c = 0;
-            if (row) {
-                for (int e = 0; e < np; e++) {
-                    const int32_t y = probe[e];
-                    c += (bit_set(row, y) && !excluded(S, ex, k, cand, y)) ? 1 : 0;
-                }
-            } else {
-                const int32_t *sa = nl <= fl ? nb : fp;
-                const int32_t *lb = nl <= fl ? fp : nb;
-                const int ns = min(nl, fl), nlong = max(nl, fl);
-                if (nlong >= a.linear_below && merge_pays(ns, nlong)) {
-                    merge_walk(sa, 0, ns, lb, nlong, [&](int32_t y) {
-                        c += excluded(S, ex, k, cand, y) ? 0 : 1;
-                    });
-                } else {
-                    for (int e = 0; e < ns; e++) {
-                        const int32_t y = sa[e];
-                        c += (contains(lb, nlong, y, a.linear_below) &&
-                              !excluded(S, ex, k, cand, y))
-                                 ? 1
-                                 : 0;
-                    }
-                }
-            }
-            lv[p - pb] = c;
-        }
-        for (int x = 0; x < P.iep_num; x++) {
-            const int p = P.iep_prefix[x];
-            const bool here = P.p_level[p] == k;
-            if (P.p_kind[p] == GAT_SET_COUNT) {
-                val[x] = here ? lv[p - pb] : (long long)S.sl[p];
-                continue;
-            }
-            const int32_t *ptr = here ? nb : S.sp[p];
-            int32_t len = here ? (int32_t)lv[p - pb] : S.sl[p];
-            const unsigned bm = P.iep_bound[x];
-            int32_t B = min_of(S, bm & ~kbit);
-            if (bm & kbit) B = min(B, cand);
-            if (B != kInf) len = lower_serial(ptr, len, B);
-            const unsigned m = P.iep_sub[x];
-            int h = 0;
-            for (int j = 0; j < P.basic; j++)
-                if ((m >> j) & 1u)
-                    h += contains(ptr, len, j == k ? cand : S.v[j], a.linear_below) ? 1 : 0;
-            val[x] = (long long)len - h;
-        }
-        unsigned long long local = 0, cur = 1;
-        int last = -1;
-        for (int g = 0; g < P.num_terms; g++) {
-            const unsigned long long v = (unsigned long long)val[P.t_slot[g]];
-            cur = (g == last + 1) ? v : cur * v;
-            if (P.t_close[g]) {
-                last = g;
-                local += cur * (unsigned long long)(long long)P.t_coef[g];
-            }
-        }
-        sum += local;
+        sum += lane_candidate<STATS>(st, P, a, k, cand, i, hit, by);
     }
     if (STATS) {
         by = t.sum(by);
         if (t.lane == 0) bytes += by;
     }
     return t.sum(sum);
+}
+
+// Two-level plans (the triangle, stars and the other patterns whose basic
+// vertices are one edge): the lanes take the level-1 units of [start, end)
+// one each, whatever their rows, so short rows leave no lane idle.  Units
+// with lists far longer than the tile's average are formed by the tile.
+template <int G, bool STATS>
+__device__ __forceinline__ void run_pairs(const Tile<G> &t, TileSmem &S, const GatPlan &P,
+                                          const SearchArgs &a, int64_t start, int64_t end,
+                                          int32_t *scratch, unsigned long long &acc,
+                                          unsigned long long &bytes) {
+    const int64_t *task_off = P.level1_bounded ? a.lo_off : a.off;
+    int32_t row = tile_bound<G, true, int64_t>(t, task_off, a.V + 1, start) - 1;
+    unsigned long long sum = 0, by = 0;
+    for (int64_t base = start; base < end; base += G) {
+        const int64_t u = base + t.lane;
+        int32_t v1 = 0, cost = 0;
+        int i = 0;
+        bool live = u < end, hit = false;
+        PairState st{0, 0, 0, nullptr};
+        if (live) {
+            // the row holding unit u: gallop from the last row, then bisect
+            int32_t step = 1;
+            while (row + step < a.V && task_off[row + step] <= u) {
+                row += step;
+                step <<= 1;
+            }
+            int32_t n = min(row + step, a.V) - row;
+            while (n > 1) {
+                const int32_t h = n >> 1;
+                if (task_off[row + h] <= u) {
+                    row += h;
+                    n -= h;
+                } else {
+                    n = h;
+                }
+            }
+            const int64_t o = a.off[row];
+            i = (int)(u - task_off[row]);
+            st.v0 = row;
+            st.d0 = (int32_t)(a.off[row + 1] - o);
+            st.lo0 = (int32_t)(a.lo_off[row + 1] - a.lo_off[row]);
+            st.nb0 = a.adj + o;
+            v1 = st.nb0[i];
+            cost = lane_cost(st, P, 1, (int32_t)(a.off[v1 + 1] - a.off[v1]));
+        }
+        unsigned heavy = heavy_lanes(t, cost);
+        if (live && !((heavy >> t.lane) & 1u))
+            sum += lane_candidate<STATS>(st, P, a, 1, v1, i, hit, by);
+        while (heavy) {
+            const int j = __ffs(heavy) - 1;
+            heavy &= heavy - 1;
+            const int32_t c0 = t.bcast(st.v0, j), c1 = t.bcast(v1, j);
+            const int ci = t.bcast(i, j);
+            t.sync();
+            if (t.lane == 0) {
+                S.v[0] = c0;
+                S.v[1] = c1;
+            }
+            t.sync();
+            level_sets<G, STATS>(t, S, P, a, 0, c0, false, scratch, bytes);
+            level_sets<G, STATS>(t, S, P, a, 1, c1, false, scratch, bytes, ci);
+            const long long r = iep_value(t, S, P, a.linear_below);
+            if (t.lane == 0) acc += (unsigned long long)r;
+            t.sync();
+        }
+    }
+    if (STATS) {
+        by = t.sum(by);
+        if (t.lane == 0) bytes += by;
+    }
+    sum = t.sum(sum);
+    if (t.lane == 0) acc += sum;
 }
 
 // The lane path pays when the candidates fill at least half the tile, or
@@ -757,6 +907,10 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
                                           int32_t *scratch, unsigned long long &acc,
                                           unsigned long long &bytes) {
     const int basic = P.basic;
+    if (!ALL_ENTRIES && basic == 2 && P.lane_last) {
+        run_pairs<G, STATS>(t, S, P, a, start, end, scratch, acc, bytes);
+        return;
+    }
     const int64_t *task_off = (!ALL_ENTRIES && P.level1_bounded) ? a.lo_off : a.off;
     int32_t row = tile_bound<G, true, int64_t>(t, task_off, a.V + 1, start) - 1;
     int32_t cur_v0 = -1;
@@ -771,18 +925,6 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
             level_sets<G, STATS>(t, S, P, a, 0, v0, false, scratch, bytes);
             cur_v0 = v0;
         }
-        if (!ALL_ENTRIES && basic == 2 && P.lane_last) {
-            // Two-level plan: the lanes take this row's units of the chunk.
-            const int64_t row_end = min(end, task_off[v0 + 1]);
-            const int i0 = (int)(tk - task_off[v0]), i1 = (int)(row_end - task_off[v0]);
-            if (lane_worth<G>(S, P, 1, i1 - i0)) {
-                const unsigned long long r = lane_last_level<G, STATS>(
-                    t, S, P, a, 1, bytes, a.adj + a.off[v0], i0, i1);
-                if (t.lane == 0) acc += r;
-                tk = row_end - 1;
-                continue;
-            }
-        }
         if (t.lane == 0) S.v[1] = v1;
         t.sync();
         level_sets<G, STATS>(t, S, P, a, 1, v1, false, scratch, bytes,
@@ -796,7 +938,7 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
         setup_level(t, S, P, 2);
         if (basic == 3 && P.lane_last && lane_worth<G>(S, P, 2, S.cnt[2])) {
             const unsigned long long r =
-                lane_last_level<G, STATS>(t, S, P, a, 2, bytes, S.src[2], 0, S.cnt[2]);
+                lane_last_level<G, STATS>(t, S, P, a, 2, bytes, S.src[2], S.cnt[2]);
             if (t.lane == 0) acc += r;
             continue;
         }
@@ -832,7 +974,7 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
             setup_level(t, S, P, k + 1);
             if (k + 1 == basic - 1 && P.lane_last && lane_worth<G>(S, P, k + 1, S.cnt[k + 1])) {
                 const unsigned long long r = lane_last_level<G, STATS>(
-                    t, S, P, a, k + 1, bytes, S.src[k + 1], 0, S.cnt[k + 1]);
+                    t, S, P, a, k + 1, bytes, S.src[k + 1], S.cnt[k + 1]);
                 if (t.lane == 0) acc += r;
                 continue;
             }
@@ -841,8 +983,26 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
     }
 }
 
+// Units of one queue grab.  A grab is at most `most` units (the configured
+// chunk), and shrinks with the units left to 1/share of a tile's part of
+// them: neighbouring units of hub rows are the heaviest, and a tile that
+// holds several of them runs on alone.  Grabbing unit by unit costs one
+// atomic and one row search each, which is cheap next to the walk under a
+// unit; counts of 12k to 2M units were all fastest at grabs of one
+// (6-cycle with chord on R-MAT 2^10 35.4 ms at 8 units a grab, 5.5 ms at 1;
+// two-level diamond on R-MAT 2^17 6.4 ms at 8 units a lane, 1.2 ms at 1).
+constexpr int kPairShare = 16;  // two-level plans: units of G at a time
+constexpr int kDeepShare = 64;
+
+__host__ __device__ __forceinline__ int64_t grab_units(int64_t left, int64_t tiles, bool pairs,
+                                                       int tile, int64_t most) {
+    const int64_t unit = pairs ? tile : 1;
+    const int64_t c = left / (tiles * (pairs ? kPairShare : kDeepShare)) / unit * unit;
+    return c < unit ? unit : (c > most ? most : c);
+}
+
 template <int G, bool STATS, bool ALL_ENTRIES = false>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
     search_kernel(const SearchArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Tile<G> t;
@@ -854,14 +1014,19 @@ __global__ void __launch_bounds__(256)
         a.scratch + ((int64_t)blockIdx.x * tiles_per_block + tile_in_block) *
                         a.scratch_stride;
     unsigned long long acc = 0, bytes = 0;
+    const bool pairs = !ALL_ENTRIES && P.basic == 2 && P.lane_last;
+    const int64_t tiles = (int64_t)gridDim.x * tiles_per_block;
+    int64_t left = a.num_tasks - a.task_begin;
     for (;;) {
         unsigned long long start = 0;
+        const int64_t take = grab_units(left, tiles, pairs, G, a.chunk);
         if (t.lane == 0)
             start = (unsigned long long)a.task_begin +
-                    atomicAdd(&a.ctr->cursor, (unsigned long long)a.chunk);
+                    atomicAdd(&a.ctr->cursor, (unsigned long long)take);
         start = t.bcast(start, 0);
         if (start >= (unsigned long long)a.num_tasks) break;
-        const int64_t end = min((int64_t)start + a.chunk, a.num_tasks);
+        left = a.num_tasks - (int64_t)start;
+        const int64_t end = min((int64_t)start + take, a.num_tasks);
         run_units<G, STATS, ALL_ENTRIES>(t, S, P, a, (int64_t)start, end, scratch, acc,
                                          bytes);
     }
@@ -871,17 +1036,16 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// Many (pattern, graph) jobs in one persistent launch.  Job j owns the
-// virtual unit range [vstart[j], vstart[j] + its units rounded up to a whole
-// chunk), so a chunk never straddles two jobs; one atomic cursor walks the
-// concatenated ranges.  A tile adds its running total to the job's result
-// whenever it moves to another job, and at exit.
+// Many (pattern, graph) jobs in one persistent launch.  The queue is counted
+// in grabs: job j owns the grabs [vstart[j], vstart[j+1]), each of its own
+// number of units, so a grab never straddles two jobs.  A tile adds its
+// running total to the job's result whenever it moves to another job, and at
+// exit.
 template <int G>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
     batch_kernel(const BatchJob *__restrict__ jobs, const int64_t *__restrict__ vstart,
-                 int32_t num_jobs, int64_t vtotal, int32_t chunk,
-                 unsigned long long *cursor, unsigned long long *results,
-                 int32_t *scratch_all, int64_t scratch_stride) {
+                 int32_t num_jobs, int64_t vtotal, unsigned long long *cursor,
+                 unsigned long long *results, int32_t *scratch_all, int64_t scratch_stride) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Tile<G> t;
     const int tiles_per_block = blockDim.x / G;
@@ -893,23 +1057,22 @@ __global__ void __launch_bounds__(256)
     int cur_job = -1;
     for (;;) {
         unsigned long long vs = 0;
-        if (t.lane == 0) vs = atomicAdd(cursor, (unsigned long long)chunk);
+        if (t.lane == 0) vs = atomicAdd(cursor, 1ull);
         vs = t.bcast(vs, 0);
         if (vs >= (unsigned long long)vtotal) break;
         const int j = tile_bound<G, true, int64_t>(t, vstart, num_jobs, (int64_t)vs) - 1;
         const BatchJob &job = jobs[j];
-        const int64_t start = job.args.task_begin + ((int64_t)vs - vstart[j]);
-        if (start >= job.args.num_tasks) continue;  // padding of the job's last chunk
+        const int64_t start = job.args.task_begin + ((int64_t)vs - vstart[j]) * job.args.chunk;
         if (j != cur_job) {
-            if (t.lane == 0 && cur_job >= 0 && acc) atomicAdd(&results[cur_job], acc);
+            if (t.lane == 0 && cur_job >= 0 && acc) atomicAdd(&results[jobs[cur_job].result], acc);
             acc = 0;
             cur_job = j;
         }
-        const int64_t end = min(start + chunk, job.args.num_tasks);
+        const int64_t end = min(start + job.args.chunk, job.args.num_tasks);
         run_units<G, false, false>(t, S, *job.args.plan, job.args, start, end, scratch, acc,
                                    bytes);
     }
-    if (t.lane == 0 && cur_job >= 0 && acc) atomicAdd(&results[cur_job], acc);
+    if (t.lane == 0 && cur_job >= 0 && acc) atomicAdd(&results[jobs[cur_job].result], acc);
 }
 
 template <int G, bool STATS>
@@ -982,9 +1145,10 @@ size_t tile_smem_bytes() { return sizeof(TileSmem); }
 size_t batch_job_bytes() { return sizeof(BatchJob); }
 
 void batch_fill_job(void *dst, const GatPlan *d_plan, const GatPlan &h_plan,
-                    const DevGraphView &g, int linear_below, bool use_bitmaps, int shard,
-                    int num_shards) {
+                    const DevGraphView &g, int linear_below, bool use_bitmaps, int result,
+                    int shard, int num_shards) {
     BatchJob j{};
+    j.result = result;
     SearchArgs &a = j.args;
     a.plan = d_plan;
     a.off = g.off;
@@ -1008,17 +1172,25 @@ int64_t batch_job_tasks(const void *job) {
     return a.num_tasks - a.task_begin;
 }
 
+int64_t batch_job_grabs(void *job, const GatPlan &plan, int64_t tiles, int tile, int chunk) {
+    SearchArgs &a = reinterpret_cast<BatchJob *>(job)->args;
+    const bool pairs = plan.basic == 2 && plan.lane_last;
+    const int64_t n = a.num_tasks - a.task_begin;
+    a.chunk = (int32_t)grab_units(n, tiles, pairs, tile, int64_t(chunk) * (pairs ? tile : 1));
+    return (n + a.chunk - 1) / a.chunk;
+}
+
 namespace {
 template <int G>
 cudaError_t batch_launch_g(const BatchJob *jobs, const int64_t *vstart, int32_t num_jobs,
-                           int64_t vtotal, int grid, int block, int chunk,
-                           unsigned long long *cursor, unsigned long long *results,
-                           int32_t *scratch, int64_t stride, cudaStream_t st) {
+                           int64_t vtotal, int grid, int block, unsigned long long *cursor,
+                           unsigned long long *results, int32_t *scratch, int64_t stride,
+                           cudaStream_t st) {
     // The shared-memory attribute is set by batch_blocks_per_sm, which callers
     // run first (outside any stream capture).
     const size_t smem = size_t(block / G) * sizeof(TileSmem);
-    batch_kernel<G><<<grid, block, smem, st>>>(jobs, vstart, num_jobs, vtotal, chunk, cursor,
-                                               results, scratch, stride);
+    batch_kernel<G><<<grid, block, smem, st>>>(jobs, vstart, num_jobs, vtotal, cursor, results,
+                                               scratch, stride);
     return cudaGetLastError();
 }
 template <int G>
@@ -1047,12 +1219,12 @@ int batch_blocks_per_sm(int tile, int block) {
 }
 
 cudaError_t launch_batch(const void *d_jobs, const int64_t *d_vstart, int32_t num_jobs,
-                         int64_t vtotal, int tile, int grid, int block, int chunk,
+                         int64_t vtotal, int tile, int grid, int block,
                          unsigned long long *d_cursor, unsigned long long *d_results,
                          int32_t *scratch, int64_t stride, cudaStream_t st) {
     const BatchJob *jobs = reinterpret_cast<const BatchJob *>(d_jobs);
 #define GAT_BL(G)                                                                        \
-    return batch_launch_g<G>(jobs, d_vstart, num_jobs, vtotal, grid, block, chunk, d_cursor, \
+    return batch_launch_g<G>(jobs, d_vstart, num_jobs, vtotal, grid, block, d_cursor, \
                              d_results, scratch, stride, st)
     switch (tile) {
         case 1: GAT_BL(1);

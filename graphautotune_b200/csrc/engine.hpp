@@ -49,7 +49,7 @@ struct LaunchShape {
     int grid = 0;         // CTAs
     int block = 128;      // threads per CTA
     int tile = 32;        // lanes cooperating on one unit
-    int chunk = 16;       // level-1 units taken per queue grab
+    int chunk = 16;       // most level-1 units taken per queue grab
     int linear_below = 0; // lists shorter than this are scanned linearly
     int64_t task_begin = 0;  // level-1 unit range [task_begin, task_end);
     int64_t task_end = -1;   // -1: all units
@@ -140,18 +140,22 @@ cudaError_t pairs_csr_device(const int32_t *pairs, int64_t n, int32_t V, int64_t
                              int32_t **adj, int64_t pad_ints, int64_t *E, cudaStream_t st);
 
 // Batched launches: host code fills an array of batch_job_bytes()-sized job
-// records (one per (plan, graph) pair), copies it and the chunk-aligned
-// virtual start of every job to the device, and launches one persistent
-// kernel over all of them.  `results` receives one signed 64-bit raw total
-// per job; cursor and results must be zero before the launch.
+// records (one per (plan, graph) pair), splits each into queue grabs
+// (batch_job_grabs), copies the records and every job's first grab to the
+// device, and launches one persistent kernel over all of them.  results[r]
+// receives the signed 64-bit raw total of the job whose `result` is r;
+// cursor and results must be zero before the launch.
 size_t batch_job_bytes();
 void batch_fill_job(void *dst, const GatPlan *d_plan, const GatPlan &h_plan,
-                    const DevGraphView &g, int linear_below, bool use_bitmaps, int shard = 0,
-                    int num_shards = 0);
+                    const DevGraphView &g, int linear_below, bool use_bitmaps, int result,
+                    int shard = 0, int num_shards = 0);
 int64_t batch_job_tasks(const void *job);
+// Fixes the job's units per grab (at most `chunk`, per lane for two-level
+// plans) on `tiles` resident tiles; returns the job's grabs.
+int64_t batch_job_grabs(void *job, const GatPlan &plan, int64_t tiles, int tile, int chunk);
 int batch_blocks_per_sm(int tile, int block);
 cudaError_t launch_batch(const void *d_jobs, const int64_t *d_vstart, int32_t num_jobs,
-                         int64_t vtotal, int tile, int grid, int block, int chunk,
+                         int64_t vtotal, int tile, int grid, int block,
                          unsigned long long *d_cursor, unsigned long long *d_results,
                          int32_t *scratch, int64_t stride, cudaStream_t st);
 

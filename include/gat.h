@@ -126,9 +126,10 @@ typedef struct gat_config {
     int32_t threads_per_warp;      /* lanes per unit: 1,2,4,8,16,32 */
     int32_t max_regs;              /* accepted for compatibility; register
                                       use is fixed when the library is built */
-    int32_t chunk;                 /* level-1 units per work-queue grab (per
-                                      lane for two-level plans, whose lanes
-                                      take units one each) */
+    int32_t chunk;                 /* most level-1 units per work-queue grab
+                                      (per lane for two-level plans, whose
+                                      lanes take units one each); grabs
+                                      shrink with the units left */
     int32_t hub_bitmaps;           /* 1: intersect against the graph's hub
                                       bitmaps where cheaper; 0: never */
     int64_t memory_budget;         /* bytes of set scratch the executor may
@@ -290,8 +291,8 @@ int gat_executor_count_shard_balg(gat_executor *e, gat_graph *g,
  * No single reference counterpart: the reference runs one pm process per
  * (pattern, graph, config) (tuning/tuning/role/driver.py:88-132).  A batch
  * counts many (schedule, graph) jobs of uneven size in ONE persistent launch:
- * the jobs' level-1 work queues are concatenated (each rounded up to a whole
- * chunk) and drained by one atomic cursor, so small jobs do not leave the GPU
+ * the jobs' level-1 work queues are split into grabs, concatenated (jobs of
+ * the most levels and longest rows first) and drained by one atomic cursor, so small jobs do not leave the GPU
  * idle.  gat_batch_prepare fixes the launch shape from `c`, uploads graphs
  * that are not resident yet, builds the job table and, with use_cuda_graph,
  * captures memset + launch + result copy into a CUDA graph that
