@@ -213,7 +213,9 @@ int gat_graph_csr(const gat_graph *g, const int64_t **offsets,
 int gat_graph_upload(gat_graph *g, int flags, void *stream);
 /* As gat_graph_upload, also building hub bitmaps: one V-bit row (bit x set
  * iff x is a neighbour) for every vertex of degree >= hub_min_degree, largest
- * degree first, as many as fit in hub_max_bytes (0 disables).
+ * degree first, as many as fit in hub_max_bytes (0 disables).  Vertices below
+ * that degree get rows too while all rows stay within 64 MiB (and
+ * hub_max_bytes); gat_graph_hubs does not count those.
  * gat_graph_upload uses the defaults below.  With GAT_UPLOAD_DEGREE_ORDER,
  * the given-id copy's bitmaps (used only by reference-compatible counts) are
  * built on first use, with these parameters. */
