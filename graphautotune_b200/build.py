@@ -64,7 +64,7 @@ def _compile(src: Path, force: bool) -> Path:
     return obj
 
 
-LIB_SOURCES = ["schedule.cpp", "plan.cpp", "graph.cpp", "capi.cpp", "engine.cu"]
+LIB_SOURCES = ["schedule.cpp", "plan.cpp", "graph.cpp", "devmem.cpp", "capi.cpp", "engine.cu"]
 
 
 def build(force: bool = False, jobs: int = 0) -> Path:

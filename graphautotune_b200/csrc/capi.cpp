@@ -8,10 +8,12 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <numeric>
 #include <string>
 
 #include "../../include/gat.h"
+#include "devmem.hpp"
 #include "engine.hpp"
 #include "gat_internal.hpp"
 #include "graph.hpp"
@@ -61,21 +63,25 @@ struct DevCopy {
     int64_t lo_total = 0;
     int32_t max_degree = 0;
     int32_t max_lower = 0;  // longest lower list (entries below the row's vertex)
+    int64_t heavy_rows = 0;  // leading rows of degree >= kC4HeavyDegree
     bool ready = false;
-    std::vector<int64_t> lo_host;   // host copy of lo_off
-    std::vector<int64_t> off_host;  // host copy of off
+    // Host copies of off and lo_off, read back when a range or a shard first
+    // asks for them (host_offsets).
+    std::mutex host_mu;
+    bool host_ready = false;
+    std::vector<int64_t> lo_host, off_host;
     int32_t *hub_slot = nullptr;    // per vertex: bitmap row or -1
     int32_t *hubs = nullptr;        // row -> vertex
     uint32_t *bitmaps = nullptr;
     int32_t nhubs = 0;
     int64_t bitmap_words = 0;
     void release() {
-        cudaFree(off);
-        cudaFree(adj);
-        cudaFree(lo_off);
-        cudaFree(hub_slot);
-        cudaFree(hubs);
-        cudaFree(bitmaps);
+        dev_free(off);
+        dev_free(adj);
+        dev_free(lo_off);
+        dev_free(hub_slot);
+        dev_free(hubs);
+        dev_free(bitmaps);
         hub_slot = nullptr;
         hubs = nullptr;
         bitmaps = nullptr;
@@ -87,13 +93,16 @@ struct DevCopy {
         lo_total = 0;
         max_degree = 0;
         max_lower = 0;
+        heavy_rows = 0;
         ready = false;
+        host_ready = false;
         lo_host.clear();
         off_host.clear();
     }
 };
 
 struct gat_graph {
+    PoolUser pool;  // freed after the copies below
     HostGraph host;
     DevCopy dev;          // ids as given
     DevCopy dev_ordered;  // relabelled by decreasing degree
@@ -115,6 +124,7 @@ struct gat_graph {
 };
 
 struct gat_executor {
+    PoolUser pool;
     gat_config cfg{};
     int device = 0;
     int sms = 0;
@@ -557,57 +567,74 @@ namespace {
 constexpr int64_t kAdjPadInts = 4;
 int64_t adj_alloc_ints(int64_t E) { return E + kAdjPadInts; }
 
-// Completes a device copy whose off and adj are in place: lo_off is derived
-// on the device, and both offset arrays are kept on the host too (range and
-// shard arithmetic reads them).  `off_known` is the host's copy of off when
-// there is one; otherwise off is read back.
-int finish_copy(DevCopy &d, int32_t V, int32_t max_degree, const std::vector<int64_t> *off_known,
-                cudaStream_t st) {
+// A copy that failed half-way: its work may still be on the stream.
+void abandon(DevCopy &d, cudaStream_t st) {
+    cudaStreamSynchronize(st);
+    d.release();
+}
+
+// Completes a device copy whose off and adj are in place: lo_off and the
+// rows' extremes are derived on the device.
+int finish_copy(DevCopy &d, int32_t V, cudaStream_t st) {
     cudaError_t e;
-    if ((e = cudaMalloc(&d.lo_off, sizeof(int64_t) * (size_t(V) + 1))) != cudaSuccess) {
-        d.release();
+    CsrExtremes *dx = nullptr, x{};
+    if ((e = dev_alloc((void **)&d.lo_off, sizeof(int64_t) * (size_t(V) + 1), st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&dx, sizeof(CsrExtremes), st)) != cudaSuccess) {
+        abandon(d, st);
+        dev_free(dx, st);
         return fail(GAT_ERR_MEMORY, std::string("device graph allocation: ") + cudaGetErrorString(e));
     }
-    d.lo_host.resize(size_t(V) + 1);
-    if (off_known)
-        d.off_host = *off_known;
-    else
-        d.off_host.resize(size_t(V) + 1);
     if ((e = lower_offsets_device(d.off, d.adj, V, d.lo_off, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d.lo_host.data(), d.lo_off, sizeof(int64_t) * (size_t(V) + 1),
-                             cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
-        (!off_known &&
-         (e = cudaMemcpyAsync(d.off_host.data(), d.off, sizeof(int64_t) * (size_t(V) + 1),
-                              cudaMemcpyDeviceToHost, st)) != cudaSuccess) ||
+        (e = csr_extremes_device(d.off, d.lo_off, V, kC4HeavyDegree, dx, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(&x, dx, sizeof(x), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess) {
-        d.release();
+        abandon(d, st);
+        dev_free(dx, st);
         return cuda_fail(e, "graph upload");
     }
-    d.lo_total = d.lo_host[size_t(V)];
-    d.max_degree = max_degree;
-    int64_t ml = 0;
-    for (size_t v = 0; v < size_t(V); v++) ml = std::max(ml, d.lo_host[v + 1] - d.lo_host[v]);
-    d.max_lower = (int32_t)ml;
+    dev_free(dx, st);
+    d.lo_total = x.lo_total;
+    d.max_degree = x.max_degree;
+    d.max_lower = x.max_lower;
+    d.heavy_rows = x.first_light;
     d.ready = true;
+    return GAT_OK;
+}
+
+// The host copies of a device copy's offsets (threads may share a graph).
+int host_offsets(DevCopy &d, int32_t V, cudaStream_t st) {
+    std::lock_guard<std::mutex> lk(d.host_mu);
+    if (d.host_ready) return GAT_OK;
+    d.off_host.resize(size_t(V) + 1);
+    d.lo_host.resize(size_t(V) + 1);
+    const size_t bytes = sizeof(int64_t) * (size_t(V) + 1);
+    cudaError_t e;
+    if ((e = cudaMemcpyAsync(d.off_host.data(), d.off, bytes, cudaMemcpyDeviceToHost, st)) !=
+            cudaSuccess ||
+        (e = cudaMemcpyAsync(d.lo_host.data(), d.lo_off, bytes, cudaMemcpyDeviceToHost, st)) !=
+            cudaSuccess ||
+        (e = cudaStreamSynchronize(st)) != cudaSuccess)
+        return cuda_fail(e, "offset read-back");
+    d.host_ready = true;
     return GAT_OK;
 }
 
 int upload_copy(const HostGraph &h, DevCopy &d, cudaStream_t st) {
     d.release();
     cudaError_t e;
-    if ((e = cudaMalloc(&d.off, sizeof(int64_t) * (h.V + 1))) != cudaSuccess ||
-        (e = cudaMalloc(&d.adj, sizeof(int32_t) * adj_alloc_ints(h.E))) != cudaSuccess) {
-        d.release();
+    if ((e = dev_alloc((void **)&d.off, sizeof(int64_t) * (h.V + 1), st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&d.adj, sizeof(int32_t) * adj_alloc_ints(h.E), st)) != cudaSuccess) {
+        abandon(d, st);
         return fail(GAT_ERR_MEMORY, std::string("device graph allocation: ") + cudaGetErrorString(e));
     }
     if ((e = cudaMemcpyAsync(d.off, h.off.data(), sizeof(int64_t) * (h.V + 1),
                              cudaMemcpyHostToDevice, st)) != cudaSuccess ||
         (h.E > 0 && (e = cudaMemcpyAsync(d.adj, h.adj.data(), sizeof(int32_t) * h.E,
                                          cudaMemcpyHostToDevice, st)) != cudaSuccess)) {
-        d.release();
+        abandon(d, st);
         return cuda_fail(e, "graph upload");
     }
-    return finish_copy(d, h.V, h.max_degree(), &h.off, st);
+    return finish_copy(d, h.V, st);
 }
 
 // The degree-ordered copy, derived on the device from the resident copy
@@ -621,24 +648,24 @@ int derive_ordered_copy(const HostGraph &h, const DevCopy &src, DevCopy &d, cuda
     }
     d.release();
     cudaError_t e;
-    if ((e = cudaMalloc(&d.off, sizeof(int64_t) * (h.V + 1))) != cudaSuccess ||
-        (e = cudaMalloc(&d.adj, sizeof(int32_t) * adj_alloc_ints(h.E))) != cudaSuccess) {
-        d.release();
+    if ((e = dev_alloc((void **)&d.off, sizeof(int64_t) * (h.V + 1), st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&d.adj, sizeof(int32_t) * adj_alloc_ints(h.E), st)) != cudaSuccess) {
+        abandon(d, st);
         return fail(GAT_ERR_MEMORY, std::string("device graph allocation: ") + cudaGetErrorString(e));
     }
-    const int32_t md = h.max_degree();
-    if ((e = relabel_by_degree_device(src.off, src.adj, h.V, h.E, md, d.off, d.adj, st)) !=
+    if ((e = relabel_by_degree_device(src.off, src.adj, h.V, h.E, src.max_degree, d.off,
+                                      d.adj, st)) !=
         cudaSuccess) {
-        d.release();
+        abandon(d, st);
         return cuda_fail(e, "degree relabel");
     }
-    return finish_copy(d, h.V, md, nullptr, st);
+    return finish_copy(d, h.V, st);
 }
 
 void release_hubs(DevCopy &d) {
-    cudaFree(d.hub_slot);
-    cudaFree(d.hubs);
-    cudaFree(d.bitmaps);
+    dev_free(d.hub_slot);
+    dev_free(d.hubs);
+    dev_free(d.bitmaps);
     d.hub_slot = nullptr;
     d.hubs = nullptr;
     d.bitmaps = nullptr;
@@ -659,44 +686,57 @@ void release_hubs(DevCopy &d) {
 constexpr int64_t kSmallRowBytes = int64_t(64) << 20;
 constexpr int64_t kRowMinDegree = 8;
 
-int upload_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes,
-                cudaStream_t st) {
+int upload_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes, bool ordered,
+                const HostGraph &h, cudaStream_t st) {
     if (min_degree <= 0 || max_bytes <= 0 || V == 0) return GAT_OK;
-    const std::vector<int64_t> &off = d.off_host;
-    auto degree = [&](int32_t v) { return off[size_t(v) + 1] - off[size_t(v)]; };
     const int64_t words = (int64_t(V) + 31) / 32;
-    std::vector<int32_t> cand;
-    for (int32_t v = 0; v < V; v++)
-        if (degree(v) >= min_degree) cand.push_back(v);
-    std::stable_sort(cand.begin(), cand.end(),
-                     [&](int32_t x, int32_t y) { return degree(x) > degree(y); });
     const int64_t fit = max_bytes / (words * 4);
-    if ((int64_t)cand.size() > fit) cand.resize(size_t(fit));
-    const size_t nhubs = cand.size();
     const int64_t room = std::min(max_bytes, kSmallRowBytes) / (words * 4);
-    if ((int64_t)nhubs < room && min_degree > kRowMinDegree) {
-        for (int32_t v = 0; v < V; v++)
-            if (degree(v) >= kRowMinDegree && degree(v) < min_degree) cand.push_back(v);
-        std::stable_sort(cand.begin() + nhubs, cand.end(),
-                         [&](int32_t x, int32_t y) { return degree(x) > degree(y); });
-        if ((int64_t)cand.size() > room) cand.resize(size_t(room));
-    }
-    if (cand.empty()) return GAT_OK;
-    std::vector<int32_t> slot(size_t(V), -1);
-    for (size_t i = 0; i < cand.size(); i++) slot[cand[i]] = (int32_t)i;
     cudaError_t e;
-    const size_t bm_bytes = size_t(cand.size()) * size_t(words) * 4;
-    if ((e = cudaMalloc(&d.hub_slot, sizeof(int32_t) * V)) != cudaSuccess ||
-        (e = cudaMalloc(&d.hubs, sizeof(int32_t) * cand.size())) != cudaSuccess ||
-        (e = cudaMalloc(&d.bitmaps, bm_bytes)) != cudaSuccess)
+    // Rows in decreasing order of degree: on the degree-ordered copy the
+    // leading ids themselves, so only the counts are needed.
+    std::vector<int32_t> cand;
+    int64_t nhubs = 0, nrows = 0;
+    if (ordered) {
+        int64_t *dn = nullptr, n[2] = {0, 0};
+        if ((e = dev_alloc((void **)&dn, sizeof(n), st)) != cudaSuccess)
+            return fail(GAT_ERR_MEMORY, std::string("hub bitmap allocation: ") + cudaGetErrorString(e));
+        if ((e = leading_rows_device(d.off, V, min_degree, kRowMinDegree, dn, st)) != cudaSuccess ||
+            (e = cudaMemcpyAsync(n, dn, sizeof(n), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+            (e = cudaStreamSynchronize(st)) != cudaSuccess) {
+            dev_free(dn, st);
+            return cuda_fail(e, "hub bitmaps");
+        }
+        dev_free(dn, st);
+        nhubs = std::min(n[0], fit);
+        nrows = std::max(nhubs, n[0] < room ? std::min(std::max(n[0], n[1]), room) : 0);
+    } else {
+        auto by_degree = [&](int32_t x, int32_t y) { return h.degree(x) > h.degree(y); };
+        for (int32_t v = 0; v < V; v++)
+            if (h.degree(v) >= min_degree) cand.push_back(v);
+        std::stable_sort(cand.begin(), cand.end(), by_degree);
+        nhubs = std::min((int64_t)cand.size(), fit);
+        if ((int64_t)cand.size() < room && min_degree > kRowMinDegree) {
+            for (int32_t v = 0; v < V; v++)
+                if (h.degree(v) >= kRowMinDegree && h.degree(v) < min_degree) cand.push_back(v);
+            std::stable_sort(cand.begin() + nhubs, cand.end(), by_degree);
+            nrows = std::min((int64_t)cand.size(), room);
+        }
+        nrows = std::max(nhubs, nrows);
+        cand.resize(size_t(nrows));
+    }
+    if (nrows == 0) return GAT_OK;
+    const size_t bm_bytes = size_t(nrows) * size_t(words) * 4;
+    if ((e = dev_alloc((void **)&d.hub_slot, sizeof(int32_t) * V, st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&d.hubs, sizeof(int32_t) * size_t(nrows), st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&d.bitmaps, bm_bytes, st)) != cudaSuccess)
         return fail(GAT_ERR_MEMORY, std::string("hub bitmap allocation: ") + cudaGetErrorString(e));
-    if ((e = cudaMemcpyAsync(d.hub_slot, slot.data(), sizeof(int32_t) * V,
-                             cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-        (e = cudaMemcpyAsync(d.hubs, cand.data(), sizeof(int32_t) * cand.size(),
-                             cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+    if ((!ordered && (e = cudaMemcpyAsync(d.hubs, cand.data(), sizeof(int32_t) * cand.size(),
+                                          cudaMemcpyHostToDevice, st)) != cudaSuccess) ||
+        (e = hub_slots_device(d.hubs, (int32_t)nrows, V, ordered, d.hub_slot, st)) != cudaSuccess ||
         (e = cudaMemsetAsync(d.bitmaps, 0, bm_bytes, st)) != cudaSuccess ||
-        (e = build_hub_bitmaps(d.off, d.adj, d.hubs, (int32_t)cand.size(), words, d.bitmaps,
-                               st)) != cudaSuccess ||
+        (e = build_hub_bitmaps(d.off, d.adj, d.hubs, (int32_t)nrows, words, d.bitmaps, st)) !=
+            cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess)
         return cuda_fail(e, "hub bitmaps");
     d.nhubs = (int32_t)nhubs;
@@ -708,7 +748,7 @@ int upload_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes,
 int ensure_dev_hubs(gat_graph *g, cudaStream_t st) {
     if (!g->dev_hubs_pending || !g->dev.ready) return GAT_OK;
     g->dev_hubs_pending = false;
-    return upload_hubs(g->dev, g->host.V, g->hub_min_degree, g->hub_max_bytes, st);
+    return upload_hubs(g->dev, g->host.V, g->hub_min_degree, g->hub_max_bytes, false, g->host, st);
 }
 }  // namespace
 
@@ -738,8 +778,8 @@ int gat_graph_generate_device(int kind, double p0, double p1, double p2, double 
     } else {
         return fail(GAT_ERR_ARGUMENT, "unknown generator");
     }
-    if ((e = cudaMalloc(&d.off, sizeof(int64_t) * (size_t(V) + 1))) != cudaSuccess) {
-        d.release();
+    if ((e = dev_alloc((void **)&d.off, sizeof(int64_t) * (size_t(V) + 1), st)) != cudaSuccess) {
+        abandon(d, st);
         return fail(GAT_ERR_MEMORY, std::string("device graph allocation: ") + cudaGetErrorString(e));
     }
     if (kind == 1) {
@@ -748,7 +788,7 @@ int gat_graph_generate_device(int kind, double p0, double p1, double p2, double 
     } else {
         int32_t *pairs = nullptr;
         const size_t bytes = sizeof(int32_t) * 2 * std::max<size_t>(edges.size(), 1);
-        if ((e = cudaMalloc(&pairs, bytes)) == cudaSuccess &&
+        if ((e = dev_alloc((void **)&pairs, bytes, st)) == cudaSuccess &&
             (edges.empty() ||
              (e = cudaMemcpyAsync(pairs, edges.data(), sizeof(int32_t) * 2 * edges.size(),
                                   cudaMemcpyHostToDevice, st)) == cudaSuccess))
@@ -756,10 +796,10 @@ int gat_graph_generate_device(int kind, double p0, double p1, double p2, double 
                                  kAdjPadInts, &E, st);
         const cudaError_t f = cudaStreamSynchronize(st);
         if (e == cudaSuccess) e = f;
-        cudaFree(pairs);
+        dev_free(pairs, st);
     }
     if (e != cudaSuccess) {
-        d.release();
+        abandon(d, st);
         return cuda_fail(e, "device graph build");
     }
     HostGraph &h = g->host;
@@ -769,10 +809,10 @@ int gat_graph_generate_device(int kind, double p0, double p1, double p2, double 
     if ((e = cudaMemcpyAsync(h.off.data(), d.off, sizeof(int64_t) * (size_t(V) + 1),
                              cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess) {
-        d.release();
+        abandon(d, st);
         return cuda_fail(e, "device graph read-back");
     }
-    int rc = finish_copy(d, V, h.max_degree(), &h.off, st);
+    int rc = finish_copy(d, V, st);
     if (rc != GAT_OK) return rc;
     int dev = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
@@ -792,42 +832,44 @@ int gat_graph_from_csr_device(int32_t V, int64_t E, const int64_t *offsets,
     DevCopy &d = g->dev;
     unsigned long long *flag = nullptr;
     cudaError_t e;
-    if ((e = cudaMalloc(&d.off, sizeof(int64_t) * (size_t(V) + 1))) != cudaSuccess ||
-        (e = cudaMalloc(&d.adj, sizeof(int32_t) * adj_alloc_ints(E))) != cudaSuccess ||
-        (e = cudaMalloc(&flag, sizeof(unsigned long long))) != cudaSuccess) {
-        d.release();
-        cudaFree(flag);
+    if ((e = dev_alloc((void **)&d.off, sizeof(int64_t) * (size_t(V) + 1), st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&d.adj, sizeof(int32_t) * adj_alloc_ints(E), st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&flag, sizeof(unsigned long long), st)) != cudaSuccess) {
+        abandon(d, st);
+        dev_free(flag, st);
         return fail(GAT_ERR_MEMORY, std::string("device graph allocation: ") + cudaGetErrorString(e));
     }
     HostGraph &h = g->host;
     h.V = V;
     h.E = E;
-    h.off.assign(offsets, offsets + size_t(V) + 1);
     unsigned long long bad = ~0ull;
+    // the host's copy of the offsets is made while the device works
+    auto keep_offsets = [&] { h.off.assign(offsets, offsets + size_t(V) + 1); };
     if ((e = cudaMemcpyAsync(d.off, offsets, sizeof(int64_t) * (size_t(V) + 1),
                              cudaMemcpyHostToDevice, st)) != cudaSuccess ||
         (E > 0 && (e = cudaMemcpyAsync(d.adj, adj, sizeof(int32_t) * size_t(E),
                                        cudaMemcpyHostToDevice, st)) != cudaSuccess) ||
         (e = csr_check_device(d.off, d.adj, V, E, flag, st)) != cudaSuccess ||
+        (keep_offsets(), false) ||
         (e = cudaMemcpyAsync(&bad, flag, sizeof(bad), cudaMemcpyDeviceToHost, st)) !=
             cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess) {
-        d.release();
-        cudaFree(flag);
+        abandon(d, st);
+        dev_free(flag, st);
         return cuda_fail(e, "graph upload");
     }
-    cudaFree(flag);
+    dev_free(flag, st);
     if (V > 0 && (h.off[0] != 0 || h.off[size_t(V)] != E))
         bad = std::min<unsigned long long>(bad, kCsrOffsets);
     if (bad != ~0ull) {
         static const char *why[] = {"", "offsets not monotone or outside [0, E]",
                                     "neighbour id out of range", "self loop",
                                     "row not strictly increasing"};
-        d.release();
+        abandon(d, st);
         return fail(GAT_ERR_ARGUMENT, "invalid CSR: row " + std::to_string(bad >> 3) + ": " +
                                           why[bad & 7u]);
     }
-    int rc = finish_copy(d, V, h.max_degree(), &h.off, st);
+    int rc = finish_copy(d, V, st);
     if (rc != GAT_OK) return rc;
     int dev = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
@@ -857,7 +899,7 @@ int gat_graph_upload_ex(gat_graph *g, int flags, int64_t hub_min_degree,
     g->hub_max_bytes = hub_max_bytes;
     g->dev_hubs_pending = (flags & GAT_UPLOAD_DEGREE_ORDER) != 0;
     if (rc == GAT_OK && !g->dev_hubs_pending)
-        rc = upload_hubs(g->dev, V, hub_min_degree, hub_max_bytes, st);
+        rc = upload_hubs(g->dev, V, hub_min_degree, hub_max_bytes, false, g->host, st);
     if (rc != GAT_OK) return rc;
     if (flags & GAT_UPLOAD_DEGREE_ORDER) {
         if (g->dev_ordered.ready && g->device == dev) {
@@ -869,7 +911,7 @@ int gat_graph_upload_ex(gat_graph *g, int flags, int64_t hub_min_degree,
             if (rc == GAT_OK) rc = derive_ordered_copy(g->host, g->dev, g->dev_ordered, st);
         }
         if (rc == GAT_OK)
-            rc = upload_hubs(g->dev_ordered, V, hub_min_degree, hub_max_bytes, st);
+            rc = upload_hubs(g->dev_ordered, V, hub_min_degree, hub_max_bytes, true, g->host, st);
         if (rc != GAT_OK) return rc;
     } else {
         g->dev_ordered.release();
@@ -952,7 +994,7 @@ namespace {
 // The exact 4-cycle count through the wedge-aggregation kernels (cycles.cu):
 // per-root counts are tallied in shared memory, so the scratch is only the
 // deferred-root list and the root kernel's list cursors.
-int run_c4(gat_executor *e, const DevGraphView &view, const DevCopy &dc, int64_t vb,
+int run_c4(gat_executor *e, const DevGraphView &view, int64_t heavy_rows, int64_t vb,
            int64_t ve, LaunchShape shape, cudaStream_t strm, bool balg, uint64_t *count,
            gat_stats *stats, std::chrono::steady_clock::time_point t0) {
     const bool wide = view.max_degree >= 65536;
@@ -962,9 +1004,7 @@ int run_c4(gat_executor *e, const DevGraphView &view, const DevCopy &dc, int64_t
     // Heavy roots: the leading run of ids with degree >= kC4HeavyDegree (on a
     // degree-ordered copy, exactly the vertices of that degree) take a CTA
     // each from the start.
-    constexpr int64_t kC4HeavyDegree = 256;
-    int64_t H = 0;
-    while (H < view.V && dc.off_host[H + 1] - dc.off_host[H] >= kC4HeavyDegree) H++;
+    const int64_t H = heavy_rows;
     const int light_grid = e->sms * locc;
     const int root_grid = e->cfg.num_blocks > 0 ? std::min(e->cfg.num_blocks, e->sms * rocc)
                                                 : e->sms * rocc;
@@ -1031,13 +1071,9 @@ int run_c4(gat_executor *e, const DevGraphView &view, const DevCopy &dc, int64_t
 // The exact k-clique count through the bit-matrix kernels (cliques.cu) over
 // roots [vb, ve).  Scratch: the root cursors, and per-CTA matrix rows only
 // when the graph's longest lower list does not fit in shared memory.
-int run_clique(gat_executor *e, const DevGraphView &view, const std::vector<int64_t> &lo_host,
-               int k, int64_t ub, int64_t ue, cudaStream_t strm, bool balg, uint64_t *count,
+int run_clique(gat_executor *e, const DevGraphView &view, int64_t vb, int64_t ve, int k,
+               int64_t ub, int64_t ue, cudaStream_t strm, bool balg, uint64_t *count,
                gat_stats *stats, std::chrono::steady_clock::time_point t0) {
-    // roots whose units meet [ub, ue): from the one holding unit ub to the
-    // last one starting before ue
-    const int64_t vb = std::upper_bound(lo_host.begin(), lo_host.end(), ub) - lo_host.begin() - 1;
-    const int64_t ve = std::lower_bound(lo_host.begin(), lo_host.end(), ue) - lo_host.begin();
     int wocc = 0, cocc = 0;
     clique_blocks_per_sm(k, balg, &wocc, &cocc);
     if (wocc <= 0 || cocc <= 0) return fail(GAT_ERR_CUDA, "clique kernels do not fit on the device");
@@ -1163,6 +1199,10 @@ int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *strea
     shape.linear_below = e->cfg.set_search_type;
     shape.use_bitmaps = e->cfg.hub_bitmaps != 0;
     const bool ranged = root_begin >= 0 || num_shards > 0;
+    if (ranged) {
+        int rc = host_offsets(*dc, view.V, strm);
+        if (rc != GAT_OK) return rc;
+    }
     if (num_shards > 0) {
         if (shard < 0 || shard >= num_shards)
             return fail(GAT_ERR_ARGUMENT, "shard index out of range");
@@ -1184,7 +1224,15 @@ int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *strea
         // exactly as the plan path numbers them.
         const int64_t ub = ranged ? shape.task_begin : 0;
         const int64_t ue = ranged ? shape.task_end : view.lo_total;
-        return run_clique(e, view, dc->lo_host, plan.n, ub, ue, strm, balg, count, stats, t0);
+        // roots whose units meet [ub, ue): from the one holding unit ub to the
+        // last one starting before ue
+        int64_t vb = 0, ve = view.V;
+        if (ranged) {
+            const std::vector<int64_t> &lo = dc->lo_host;
+            vb = std::upper_bound(lo.begin(), lo.end(), ub) - lo.begin() - 1;
+            ve = std::lower_bound(lo.begin(), lo.end(), ue) - lo.begin();
+        }
+        return run_clique(e, view, vb, ve, plan.n, ub, ue, strm, balg, count, stats, t0);
     }
     if (plan.special == GAT_SPECIAL_C4 && s->mode == GAT_MODE_EXACT &&
         e->cfg.special_kernels == 1) {
@@ -1216,7 +1264,7 @@ int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *strea
             vb = first_root(total * shard / num_shards);
             ve = shard + 1 == num_shards ? view.V : first_root(total * (shard + 1) / num_shards);
         }
-        return run_c4(e, view, *dc, vb, ve, shape, strm, balg, count, stats, t0);
+        return run_c4(e, view, dc->heavy_rows, vb, ve, shape, strm, balg, count, stats, t0);
     }
     int occ = blocks_per_sm(shape.tile, shape.block, balg);
     if (occ <= 0) return fail(GAT_ERR_CUDA, "kernel does not fit on the device");
@@ -1330,6 +1378,7 @@ int gat_executor_count_shard_balg(gat_executor *e, gat_graph *g, const gat_sched
 // ------------------------------------------------------------------ batch
 
 struct gat_batch {
+    PoolUser pool;
     struct Job {
         gat_graph *g;
         const gat_schedule *s;
@@ -1358,12 +1407,12 @@ struct gat_batch {
         if (graph) cudaGraphDestroy(graph);
         exec = nullptr;
         graph = nullptr;
-        cudaFree(d_plans);
-        cudaFree(d_jobs);
-        cudaFree(d_vstart);
-        cudaFree(d_cursor);
-        cudaFree(d_results);
-        cudaFree(d_scratch);
+        dev_free(d_plans);
+        dev_free(d_jobs);
+        dev_free(d_vstart);
+        dev_free(d_cursor);
+        dev_free(d_results);
+        dev_free(d_scratch);
         cudaFreeHost(h_results);
         d_plans = nullptr;
         d_jobs = nullptr;
@@ -1440,6 +1489,16 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
     std::vector<unsigned char> host_jobs(J * jb);
     std::vector<GatPlan> plans(J);
     std::vector<int64_t> vstart(J);
+    cudaError_t e;
+    for (const gat_batch::Job &job : b->jobs) {
+        const bool exact = job.s->mode == GAT_MODE_EXACT;
+        int rc = GAT_OK;
+        if (!job.g->dev.ready || (exact && !job.g->dev_ordered.ready))
+            rc = gat_graph_upload(job.g, exact ? GAT_UPLOAD_DEGREE_ORDER : 0, b->stream);
+        if (rc == GAT_OK && !(exact && job.g->dev_ordered.ready))
+            rc = ensure_dev_hubs(job.g, b->stream);
+        if (rc != GAT_OK) return rc;
+    }
     // The queue's order: plans with more levels first, and of those the jobs
     // with the longest rows, so that a job of heavy units does not start when
     // the others are nearly done.
@@ -1448,7 +1507,7 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
     auto weight = [&](size_t j) {
         const GatPlan &p = b->jobs[j].s->plan.plan;
         return std::make_pair(p.basic, double(b->jobs[j].g->host.E) *
-                                           std::pow(double(b->jobs[j].g->host.max_degree()),
+                                           std::pow(double(b->jobs[j].g->dev.max_degree),
                                                     double(p.basic - 1)));
     };
     std::vector<std::pair<int32_t, double>> weights(J);
@@ -1457,8 +1516,7 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
                      [&](size_t x, size_t y) { return weights[x] > weights[y]; });
     b->divisors.assign(J, 1);
     b->modes.assign(J, 0);
-    cudaError_t e;
-    if ((e = cudaMalloc(&b->d_plans, sizeof(GatPlan) * J)) != cudaSuccess)
+    if ((e = dev_alloc((void **)&b->d_plans, sizeof(GatPlan) * J, b->stream)) != cudaSuccess)
         return fail(GAT_ERR_MEMORY, "batch plans");
     int64_t stride = 0;
     b->units = 0;
@@ -1467,14 +1525,6 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
         gat_graph *g = b->jobs[j].g;
         const gat_schedule *s = b->jobs[j].s;
         const bool exact = s->mode == GAT_MODE_EXACT;
-        if (!g->dev.ready || (exact && !g->dev_ordered.ready)) {
-            int rc = gat_graph_upload(g, exact ? GAT_UPLOAD_DEGREE_ORDER : 0, b->stream);
-            if (rc != GAT_OK) return rc;
-        }
-        if (!(exact && g->dev_ordered.ready)) {
-            int rc = ensure_dev_hubs(g, b->stream);
-            if (rc != GAT_OK) return rc;
-        }
         const DevCopy &dc = (exact && g->dev_ordered.ready) ? g->dev_ordered : g->dev;
         DevGraphView v;
         v.V = g->host.V;
@@ -1517,11 +1567,11 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
                                      int64_t(b->grid) * (b->block / b->tile), b->tile, b->chunk);
     }
     b->scratch_bytes = size_t(std::max<int64_t>(per_block * b->grid, 4));
-    if ((e = cudaMalloc(&b->d_jobs, J * jb)) != cudaSuccess ||
-        (e = cudaMalloc(&b->d_vstart, sizeof(int64_t) * J)) != cudaSuccess ||
-        (e = cudaMalloc(&b->d_cursor, sizeof(unsigned long long))) != cudaSuccess ||
-        (e = cudaMalloc(&b->d_results, sizeof(unsigned long long) * J)) != cudaSuccess ||
-        (e = cudaMalloc(&b->d_scratch, b->scratch_bytes)) != cudaSuccess ||
+    if ((e = dev_alloc((void **)&b->d_jobs, J * jb, b->stream)) != cudaSuccess ||
+        (e = dev_alloc((void **)&b->d_vstart, sizeof(int64_t) * J, b->stream)) != cudaSuccess ||
+        (e = dev_alloc((void **)&b->d_cursor, sizeof(unsigned long long), b->stream)) != cudaSuccess ||
+        (e = dev_alloc((void **)&b->d_results, sizeof(unsigned long long) * J, b->stream)) != cudaSuccess ||
+        (e = dev_alloc((void **)&b->d_scratch, b->scratch_bytes, b->stream)) != cudaSuccess ||
         (e = cudaMallocHost(&b->h_results, sizeof(unsigned long long) * J)) != cudaSuccess)
         return fail(GAT_ERR_MEMORY, std::string("batch tables: ") + cudaGetErrorString(e));
     if ((e = cudaMemcpyAsync(b->d_plans, plans.data(), sizeof(GatPlan) * J,

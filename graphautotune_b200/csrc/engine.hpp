@@ -37,6 +37,23 @@ cudaError_t build_hub_bitmaps(const int64_t *off, const int32_t *adj,
 // device CSR with sorted rows (relabel.cu).
 cudaError_t lower_offsets_device(const int64_t *off, const int32_t *adj, int32_t V,
                                  int64_t *lo_off, cudaStream_t stream);
+// What the host needs to know of a device CSR's rows.
+struct CsrExtremes {
+    int64_t lo_total;     // lo_off[V]
+    int32_t max_degree;
+    int32_t max_lower;    // longest lower list
+    int32_t first_light;  // first row of degree below the limit (V if none)
+    int32_t pad;
+};
+cudaError_t csr_extremes_device(const int64_t *off, const int64_t *lo_off, int32_t V,
+                                int64_t light_below, CsrExtremes *out, cudaStream_t stream);
+// On a degree-ordered copy: out[0] rows of degree >= d0, out[1] of >= d1.
+cudaError_t leading_rows_device(const int64_t *off, int32_t V, int64_t d0, int64_t d1,
+                                int64_t *out, cudaStream_t stream);
+// slot[v] = bitmap row of v or -1.  ordered: rows 0 .. n-1 are the vertices
+// of those ids (hubs is filled), else hubs names them.
+cudaError_t hub_slots_device(int32_t *hubs, int32_t n, int32_t V, bool ordered, int32_t *slot,
+                             cudaStream_t stream);
 // Whether relabel_by_degree_device takes a graph of this size.
 bool relabel_fits_device(int32_t V, int64_t E);
 // The copy relabelled by decreasing degree (ties by id), rows sorted, built
@@ -70,6 +87,7 @@ struct DevCounters {
 // [v_begin, v_end) (plans with special == GAT_SPECIAL_C4), tallied in shared
 // memory (cycles.cu).  Roots below heavy_end take a CTA each; the others a
 // warp each, which defers roots with many wedges to the CTA kernel.
+constexpr int64_t kC4HeavyDegree = 256;  // rows that take a CTA each from the start
 struct C4Aux {
     unsigned long long light_cursor;
     unsigned long long deferred_count;

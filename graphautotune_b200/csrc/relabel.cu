@@ -13,6 +13,7 @@
 #include <climits>
 #include <initializer_list>
 
+#include "devmem.hpp"
 #include "engine.hpp"
 
 namespace gat {
@@ -78,6 +79,58 @@ __global__ void scatter_rows_kernel(const int64_t *__restrict__ off,
     for (int64_t i = lane; i < n; i += 32) out[dst + i] = nid[adj[src + i]];
 }
 
+__global__ void extremes_kernel(const int64_t *__restrict__ off,
+                                const int64_t *__restrict__ lo_off, int32_t V,
+                                int64_t light_below, CsrExtremes *out) {
+    int32_t md = 0, ml = 0, fl = V;
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < V;
+         v += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t d = off[v + 1] - off[v];
+        md = max(md, (int32_t)d);
+        ml = max(ml, (int32_t)(lo_off[v + 1] - lo_off[v]));
+        if (d < light_below) fl = min(fl, (int32_t)v);
+    }
+    md = __reduce_max_sync(0xffffffffu, md);
+    ml = __reduce_max_sync(0xffffffffu, ml);
+    fl = __reduce_min_sync(0xffffffffu, fl);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&out->max_degree, md);
+        atomicMax(&out->max_lower, ml);
+        atomicMin(&out->first_light, fl);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) out->lo_total = lo_off[V];
+}
+
+__global__ void extremes_init_kernel(int32_t V, CsrExtremes *out) {
+    *out = CsrExtremes{0, 0, 0, V, 0};
+}
+
+// Degrees never increase along a degree-ordered copy: bisection.
+__global__ void leading_rows_kernel(const int64_t *__restrict__ off, int32_t V, int64_t d0,
+                                    int64_t d1, int64_t *out) {
+    const int64_t want = threadIdx.x == 0 ? d0 : d1;
+    int64_t lo = 0, n = V;
+    while (n > 0) {
+        const int64_t h = n >> 1, v = lo + h;
+        const bool right = off[v + 1] - off[v] >= want;
+        lo = right ? v + 1 : lo;
+        n = right ? n - h - 1 : h;
+    }
+    out[threadIdx.x] = lo;
+}
+
+__global__ void hub_ids_kernel(int32_t n, int32_t V, int32_t *hubs, int32_t *slot) {
+    const int32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= V) return;
+    slot[v] = v < n ? v : -1;
+    if (v < n) hubs[v] = v;
+}
+
+__global__ void hub_scatter_kernel(const int32_t *__restrict__ hubs, int32_t n, int32_t *slot) {
+    const int32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h < n) slot[hubs[h]] = h;
+}
+
 unsigned blocks_for(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
 
 template <class F>
@@ -86,9 +139,9 @@ cudaError_t with_temp(F &&call, cudaStream_t st) {
     cudaError_t e = call(nullptr, bytes);
     if (e != cudaSuccess) return e;
     void *tmp = nullptr;
-    if ((e = cudaMallocAsync(&tmp, bytes ? bytes : 1, st)) != cudaSuccess) return e;
+    if ((e = dev_alloc((void **)&tmp, bytes ? bytes : 1, st)) != cudaSuccess) return e;
     e = call(tmp, bytes);
-    const cudaError_t f = cudaFreeAsync(tmp, st);
+    const cudaError_t f = dev_free(tmp, st);
     return e != cudaSuccess ? e : f;
 }
 
@@ -97,7 +150,7 @@ cudaError_t with_temp(F &&call, cudaStream_t st) {
 cudaError_t lower_offsets_device(const int64_t *off, const int32_t *adj, int32_t V,
                                  int64_t *lo_off, cudaStream_t st) {
     int64_t *cnt = nullptr;
-    cudaError_t e = cudaMallocAsync(&cnt, sizeof(int64_t) * (size_t(V) + 1), st);
+    cudaError_t e = dev_alloc((void **)&cnt, sizeof(int64_t) * (size_t(V) + 1), st);
     if (e != cudaSuccess) return e;
     lower_count_kernel<<<blocks_for(int64_t(V) + 1, 256), 256, 0, st>>>(off, adj, V, cnt);
     e = cudaGetLastError();
@@ -107,8 +160,34 @@ cudaError_t lower_offsets_device(const int64_t *off, const int32_t *adj, int32_t
                 return cub::DeviceScan::ExclusiveSum(t, b, cnt, lo_off, V + 1, st);
             },
             st);
-    const cudaError_t f = cudaFreeAsync(cnt, st);
+    const cudaError_t f = dev_free(cnt, st);
     return e != cudaSuccess ? e : f;
+}
+
+cudaError_t csr_extremes_device(const int64_t *off, const int64_t *lo_off, int32_t V,
+                                int64_t light_below, CsrExtremes *out, cudaStream_t st) {
+    extremes_init_kernel<<<1, 1, 0, st>>>(V, out);
+    extremes_kernel<<<V < (1 << 20) ? blocks_for(int64_t(V) + 1, 256) : 4096, 256, 0, st>>>(
+        off, lo_off, V, light_below, out);
+    return cudaGetLastError();
+}
+
+cudaError_t leading_rows_device(const int64_t *off, int32_t V, int64_t d0, int64_t d1,
+                                int64_t *out, cudaStream_t st) {
+    leading_rows_kernel<<<1, 2, 0, st>>>(off, V, d0, d1, out);
+    return cudaGetLastError();
+}
+
+cudaError_t hub_slots_device(int32_t *hubs, int32_t n, int32_t V, bool ordered, int32_t *slot,
+                             cudaStream_t st) {
+    if (ordered) {
+        hub_ids_kernel<<<blocks_for(V, 256), 256, 0, st>>>(n, V, hubs, slot);
+        return cudaGetLastError();
+    }
+    cudaError_t e = cudaMemsetAsync(slot, 0xFF, sizeof(int32_t) * size_t(V), st);
+    if (e != cudaSuccess) return e;
+    hub_scatter_kernel<<<blocks_for(n, 256), 256, 0, st>>>(hubs, n, slot);
+    return cudaGetLastError();
 }
 
 bool relabel_fits_device(int32_t V, int64_t E) { return V > 0 && E <= INT_MAX; }
@@ -122,13 +201,13 @@ cudaError_t relabel_by_degree_device(const int64_t *off, const int32_t *adj, int
     int64_t *ndeg = nullptr;
     const size_t nv = size_t(V);
     cudaError_t e;
-    if ((e = cudaMallocAsync(&key, 4 * nv, st)) != cudaSuccess ||
-        (e = cudaMallocAsync(&key_sorted, 4 * nv, st)) != cudaSuccess ||
-        (e = cudaMallocAsync(&id, 4 * nv, st)) != cudaSuccess ||
-        (e = cudaMallocAsync(&order, 4 * nv, st)) != cudaSuccess ||
-        (e = cudaMallocAsync(&nid, 4 * nv, st)) != cudaSuccess ||
-        (e = cudaMallocAsync(&ndeg, 8 * (nv + 1), st)) != cudaSuccess ||
-        (e = cudaMallocAsync(&unsorted, 4 * size_t(E > 0 ? E : 1), st)) != cudaSuccess) {
+    if ((e = dev_alloc((void **)&key, 4 * nv, st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&key_sorted, 4 * nv, st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&id, 4 * nv, st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&order, 4 * nv, st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&nid, 4 * nv, st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&ndeg, 8 * (nv + 1), st)) != cudaSuccess ||
+        (e = dev_alloc((void **)&unsorted, 4 * size_t(E > 0 ? E : 1), st)) != cudaSuccess) {
         // fall through to the frees
     } else {
         degree_key_kernel<<<blocks_for(V, 256), 256, 0, st>>>(off, V, max_degree, key, id);
@@ -169,7 +248,7 @@ cudaError_t relabel_by_degree_device(const int64_t *off, const int32_t *adj, int
     for (void *p : {(void *)key, (void *)key_sorted, (void *)id, (void *)order, (void *)nid,
                     (void *)ndeg, (void *)unsorted})
         if (p) {
-            const cudaError_t f = cudaFreeAsync(p, st);
+            const cudaError_t f = dev_free(p, st);
             if (e == cudaSuccess) e = f;
         }
     return e;

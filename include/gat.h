@@ -206,7 +206,8 @@ int gat_graph_csr(const gat_graph *g, const int64_t **offsets,
                   const int32_t **adj);
 /* Copies the graph to the current device (GlobalMemoryGraph::to_device,
  * graph_backend.cuh:102-118; the device copy is owned and freed by the
- * handle).  flags: GAT_UPLOAD_DEGREE_ORDER also builds a copy relabelled by
+ * handle, into a library pool that keeps up to 2 GiB per device mapped while
+ * the process holds any graph, executor or batch).  flags: GAT_UPLOAD_DEGREE_ORDER also builds a copy relabelled by
  * decreasing degree, which exact-mode counts use (exact counts do not depend
  * on vertex ids; reference-compatible counts always use the ids as given). */
 #define GAT_UPLOAD_DEGREE_ORDER 1
