@@ -1082,9 +1082,10 @@ int run_clique(gat_executor *e, const DevGraphView &view, int64_t vb, int64_t ve
                                                : e->sms * cocc;
     auto al = [](int64_t b) { return (b + 255) / 256 * 256; };
     const int64_t aux_bytes = al(sizeof(CliqueAux));
-    const int64_t stride = clique_rows_words(view.max_lower);
+    const int64_t stride = clique_rows_words(k, view.max_lower);
     const int64_t rows_bytes = al(int64_t(cta_grid) * stride * 4);
-    const size_t need = size_t(aux_bytes + rows_bytes);
+    const int64_t list_bytes = al(clique_list_ints(view.lo_total) * 4);
+    const size_t need = size_t(aux_bytes + list_bytes + rows_bytes);
     cudaError_t ce;
     if (need > e->scratch_bytes) {
         cudaFree(e->scratch);
@@ -1107,7 +1108,8 @@ int run_clique(gat_executor *e, const DevGraphView &view, int64_t vb, int64_t ve
     L.cta_grid = cta_grid;
     L.ctr = e->ctr;
     L.aux = reinterpret_cast<CliqueAux *>(base);
-    L.rows = stride > 0 ? reinterpret_cast<uint32_t *>(base + aux_bytes) : nullptr;
+    L.lists = reinterpret_cast<int32_t *>(base + aux_bytes);
+    L.rows = stride > 0 ? reinterpret_cast<uint32_t *>(base + aux_bytes + list_bytes) : nullptr;
     L.rows_stride = stride;
     L.stats = balg;
     cudaEventRecord(e->ev0, strm);

@@ -116,12 +116,14 @@ cudaError_t launch_c4(const C4Launch &launch, cudaStream_t st);
 // of each root's lower list (cliques.cu).  Needs lo_off, every lower list of
 // at most kCliqueMaxLower entries, and adj readable 4 ints past its end.
 // `rows` holds cta_grid slices of rows_stride words when
-// clique_rows_words(max lower degree) > 0, else it may be null.
+// clique_rows_words(k, max lower degree) > 0, else it may be null.
 constexpr int kCliqueMaxLower = 2048;
 constexpr int kCliqueCtaThreads = 512;  // threads of the CTA-per-root kernel
+constexpr int kCliqueLists = 4;  // CTA roots by length of lower list
 struct CliqueAux {
     unsigned long long warp_cursor;
     unsigned long long cta_cursor;
+    unsigned long long listed[kCliqueLists];
     unsigned long long pad[2];
 };
 struct CliqueLaunch {
@@ -134,9 +136,11 @@ struct CliqueLaunch {
     CliqueAux *aux = nullptr;
     uint32_t *rows = nullptr;
     int64_t rows_stride = 0;
+    int32_t *lists = nullptr;  // clique_list_ints(g.lo_total) ints
     bool stats = false;
 };
-int64_t clique_rows_words(int32_t max_lower);
+int64_t clique_rows_words(int k, int32_t max_lower);
+int64_t clique_list_ints(int64_t lo_total);
 void clique_blocks_per_sm(int k, bool stats, int *warp_occ, int *cta_occ);
 cudaError_t launch_clique(const CliqueLaunch &launch, cudaStream_t st);
 
