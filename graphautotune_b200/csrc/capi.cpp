@@ -64,6 +64,7 @@ struct DevCopy {
     int32_t max_degree = 0;
     int32_t max_lower = 0;  // longest lower list (entries below the row's vertex)
     int64_t heavy_rows = 0;  // leading rows of degree >= kC4HeavyDegree
+    int32_t c4_bound[4] = {}, c4_limit = 0;  // C4Launch::bound, x_limit
     bool ready = false;
     // Host copies of off and lo_off, read back when a range or a shard first
     // asks for them (host_offsets).
@@ -575,7 +576,7 @@ void abandon(DevCopy &d, cudaStream_t st) {
 
 // Completes a device copy whose off and adj are in place: lo_off and the
 // rows' extremes are derived on the device.
-int finish_copy(DevCopy &d, int32_t V, cudaStream_t st) {
+int finish_copy(DevCopy &d, int32_t V, bool ordered, cudaStream_t st) {
     cudaError_t e;
     CsrExtremes *dx = nullptr, x{};
     if ((e = dev_alloc((void **)&d.lo_off, sizeof(int64_t) * (size_t(V) + 1), st)) != cudaSuccess ||
@@ -585,7 +586,8 @@ int finish_copy(DevCopy &d, int32_t V, cudaStream_t st) {
         return fail(GAT_ERR_MEMORY, std::string("device graph allocation: ") + cudaGetErrorString(e));
     }
     if ((e = lower_offsets_device(d.off, d.adj, V, d.lo_off, st)) != cudaSuccess ||
-        (e = csr_extremes_device(d.off, d.lo_off, V, kC4HeavyDegree, dx, st)) != cudaSuccess ||
+        (e = csr_extremes_device(d.off, d.lo_off, V, kC4HeavyDegree, ordered, dx, st)) !=
+            cudaSuccess ||
         (e = cudaMemcpyAsync(&x, dx, sizeof(x), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess) {
         abandon(d, st);
@@ -597,6 +599,10 @@ int finish_copy(DevCopy &d, int32_t V, cudaStream_t st) {
     d.max_degree = x.max_degree;
     d.max_lower = x.max_lower;
     d.heavy_rows = x.first_light;
+    // Without an order of the ids the largest degree bounds them all.
+    for (int i = 0; i < 4; i++)
+        d.c4_bound[i] = ordered || x.max_degree >= (1 << (16 >> i)) ? x.below[i] : 0;
+    d.c4_limit = x.below[4];
     d.ready = true;
     return GAT_OK;
 }
@@ -619,7 +625,7 @@ int host_offsets(DevCopy &d, int32_t V, cudaStream_t st) {
     return GAT_OK;
 }
 
-int upload_copy(const HostGraph &h, DevCopy &d, cudaStream_t st) {
+int upload_copy(const HostGraph &h, DevCopy &d, bool ordered, cudaStream_t st) {
     d.release();
     cudaError_t e;
     if ((e = dev_alloc((void **)&d.off, sizeof(int64_t) * (h.V + 1), st)) != cudaSuccess ||
@@ -634,7 +640,7 @@ int upload_copy(const HostGraph &h, DevCopy &d, cudaStream_t st) {
         abandon(d, st);
         return cuda_fail(e, "graph upload");
     }
-    return finish_copy(d, h.V, st);
+    return finish_copy(d, h.V, ordered, st);
 }
 
 // The degree-ordered copy, derived on the device from the resident copy
@@ -644,7 +650,7 @@ int derive_ordered_copy(const HostGraph &h, const DevCopy &src, DevCopy &d, cuda
     if (!relabel_fits_device(h.V, h.E)) {
         HostGraph r;
         relabel_by_degree(h, r, nullptr);
-        return upload_copy(r, d, st);
+        return upload_copy(r, d, true, st);
     }
     d.release();
     cudaError_t e;
@@ -659,7 +665,7 @@ int derive_ordered_copy(const HostGraph &h, const DevCopy &src, DevCopy &d, cuda
         abandon(d, st);
         return cuda_fail(e, "degree relabel");
     }
-    return finish_copy(d, h.V, st);
+    return finish_copy(d, h.V, true, st);
 }
 
 void release_hubs(DevCopy &d) {
@@ -812,7 +818,7 @@ int gat_graph_generate_device(int kind, double p0, double p1, double p2, double 
         abandon(d, st);
         return cuda_fail(e, "device graph read-back");
     }
-    int rc = finish_copy(d, V, st);
+    int rc = finish_copy(d, V, false, st);
     if (rc != GAT_OK) return rc;
     int dev = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
@@ -869,7 +875,7 @@ int gat_graph_from_csr_device(int32_t V, int64_t E, const int64_t *offsets,
         return fail(GAT_ERR_ARGUMENT, "invalid CSR: row " + std::to_string(bad >> 3) + ": " +
                                           why[bad & 7u]);
     }
-    int rc = finish_copy(d, V, st);
+    int rc = finish_copy(d, V, false, st);
     if (rc != GAT_OK) return rc;
     int dev = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
@@ -894,7 +900,7 @@ int gat_graph_upload_ex(gat_graph *g, int flags, int64_t hub_min_degree,
     if (g->dev.ready && g->device == dev)
         release_hubs(g->dev);
     else if ((rc = ensure_host_adj(g)) == GAT_OK)
-        rc = upload_copy(g->host, g->dev, st);
+        rc = upload_copy(g->host, g->dev, false, st);
     g->hub_min_degree = hub_min_degree;
     g->hub_max_bytes = hub_max_bytes;
     g->dev_hubs_pending = (flags & GAT_UPLOAD_DEGREE_ORDER) != 0;
@@ -994,17 +1000,17 @@ namespace {
 // The exact 4-cycle count through the wedge-aggregation kernels (cycles.cu):
 // per-root counts are tallied in shared memory, so the scratch is only the
 // deferred-root list and the root kernel's list cursors.
-int run_c4(gat_executor *e, const DevGraphView &view, int64_t heavy_rows, int64_t vb,
+int run_c4(gat_executor *e, const DevGraphView &view, const DevCopy &dc, int64_t vb,
            int64_t ve, LaunchShape shape, cudaStream_t strm, bool balg, uint64_t *count,
            gat_stats *stats, std::chrono::steady_clock::time_point t0) {
-    const bool wide = view.max_degree >= 65536;
+    const int root_threads = c4_root_threads(view.E);
     const int locc = c4_light_blocks_per_sm(balg);
-    const int rocc = c4_root_blocks_per_sm(wide, balg);
+    const int rocc = c4_root_blocks_per_sm(root_threads, balg);
     if (locc <= 0 || rocc <= 0) return fail(GAT_ERR_CUDA, "4-cycle kernels do not fit on the device");
     // Heavy roots: the leading run of ids with degree >= kC4HeavyDegree (on a
     // degree-ordered copy, exactly the vertices of that degree) take a CTA
     // each from the start.
-    const int64_t H = heavy_rows;
+    const int64_t H = dc.heavy_rows;
     const int light_grid = e->sms * locc;
     const int root_grid = e->cfg.num_blocks > 0 ? std::min(e->cfg.num_blocks, e->sms * rocc)
                                                 : e->sms * rocc;
@@ -1013,7 +1019,8 @@ int run_c4(gat_executor *e, const DevGraphView &view, int64_t heavy_rows, int64_
     const int64_t aux_bytes = al(sizeof(C4Aux));
     const int64_t def_bytes = al(std::max<int64_t>(view.V, 1) * 4);
     const int64_t cur_bytes = al(int64_t(root_grid) * stride * 4);
-    const size_t need = size_t(aux_bytes + def_bytes + cur_bytes);
+    const int64_t mark_bytes = al(c4_mark_ints(view.V) * 4);
+    const size_t need = size_t(aux_bytes + def_bytes + cur_bytes + mark_bytes);
     cudaError_t ce;
     if (need > e->scratch_bytes) {
         cudaFree(e->scratch);
@@ -1032,11 +1039,15 @@ int run_c4(gat_executor *e, const DevGraphView &view, int64_t heavy_rows, int64_
     L.heavy_end = H;
     L.light_grid = light_grid;
     L.root_grid = root_grid;
+    L.root_threads = root_threads;
     L.ctr = e->ctr;
     L.aux = reinterpret_cast<C4Aux *>(base);
     L.deferred = reinterpret_cast<int32_t *>(base + aux_bytes);
     L.cursors = reinterpret_cast<int32_t *>(base + aux_bytes + def_bytes);
     L.cursor_stride = stride;
+    L.marks = reinterpret_cast<int32_t *>(base + aux_bytes + def_bytes + cur_bytes);
+    for (int i = 0; i < 4; i++) L.bound[i] = dc.c4_bound[i];
+    L.x_limit = dc.c4_limit;
     L.stats = balg;
     cudaEventRecord(e->ev0, strm);
     ce = launch_c4(L, strm);
@@ -1058,7 +1069,7 @@ int run_c4(gat_executor *e, const DevGraphView &view, int64_t heavy_rows, int64_
     st.tasks = (uint64_t)(ve - vb);
     st.balg_bytes = e->host_ctr->bytes;
     st.grid = root_grid;
-    st.block = 1024;
+    st.block = root_threads;
     st.tile = shape.tile;
     st.launches = (std::max(vb, H) < ve ? 1 : 0) + 1;
     st.scratch_bytes = (int64_t)need;
@@ -1266,7 +1277,7 @@ int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *strea
             vb = first_root(total * shard / num_shards);
             ve = shard + 1 == num_shards ? view.V : first_root(total * (shard + 1) / num_shards);
         }
-        return run_c4(e, view, dc->heavy_rows, vb, ve, shape, strm, balg, count, stats, t0);
+        return run_c4(e, view, *dc, vb, ve, shape, strm, balg, count, stats, t0);
     }
     int occ = blocks_per_sm(shape.tile, shape.block, balg);
     if (occ <= 0) return fail(GAT_ERR_CUDA, "kernel does not fit on the device");

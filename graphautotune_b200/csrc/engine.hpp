@@ -43,10 +43,12 @@ struct CsrExtremes {
     int32_t max_degree;
     int32_t max_lower;    // longest lower list
     int32_t first_light;  // first row of degree below the limit (V if none)
-    int32_t pad;
+    int32_t below[5];     // on a degree-ordered copy: first row of degree below
+                          // 2^16, 2^8, 2^4, 2^2, 2
 };
 cudaError_t csr_extremes_device(const int64_t *off, const int64_t *lo_off, int32_t V,
-                                int64_t light_below, CsrExtremes *out, cudaStream_t stream);
+                                int64_t light_below, bool ordered, CsrExtremes *out,
+                                cudaStream_t stream);
 // On a degree-ordered copy: out[0] rows of degree >= d0, out[1] of >= d1.
 cudaError_t leading_rows_device(const int64_t *off, int32_t V, int64_t d0, int64_t d1,
                                 int64_t *out, cudaStream_t stream);
@@ -97,16 +99,21 @@ struct C4Aux {
 struct C4Launch {
     DevGraphView g;
     int64_t v_begin = 0, v_end = 0, heavy_end = 0;
-    int light_grid = 0, root_grid = 0;
+    int light_grid = 0, root_grid = 0, root_threads = 0;
     DevCounters *ctr = nullptr;
     C4Aux *aux = nullptr;
     int32_t *deferred = nullptr;   // room for every light root
     int32_t *cursors = nullptr;    // root_grid x cursor_stride list positions
     int64_t cursor_stride = 0;     // >= the largest degree
+    int32_t bound[4] = {};         // from bound[i] on degrees are below 2^16, 2^8, 2^4, 2^2
+    int32_t x_limit = 0;           // from here on degrees are below 2
+    int32_t *marks = nullptr;      // c4_mark_ints(V) ints
     bool stats = false;
 };
+int64_t c4_mark_ints(int32_t V);
 int c4_light_blocks_per_sm(bool stats);
-int c4_root_blocks_per_sm(bool wide, bool stats);
+int c4_root_threads(int64_t E);  // threads of the root kernel's CTAs on this graph
+int c4_root_blocks_per_sm(int threads, bool stats);
 cudaError_t launch_c4(const C4Launch &launch, cudaStream_t st);
 
 // Exact k-clique count (4 <= k <= 7) over the level-1 units [u_begin, u_end)

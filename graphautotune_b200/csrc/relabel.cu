@@ -102,7 +102,7 @@ __global__ void extremes_kernel(const int64_t *__restrict__ off,
 }
 
 __global__ void extremes_init_kernel(int32_t V, CsrExtremes *out) {
-    *out = CsrExtremes{0, 0, 0, V, 0};
+    *out = CsrExtremes{0, 0, 0, V, {V, V, V, V, V}};
 }
 
 // Degrees never increase along a degree-ordered copy: bisection.
@@ -117,6 +117,20 @@ __global__ void leading_rows_kernel(const int64_t *__restrict__ off, int32_t V, 
         n = right ? n - h - 1 : h;
     }
     out[threadIdx.x] = lo;
+}
+
+// The bounds of the 4-cycle kernels' counter widths, likewise.
+__global__ void degree_bounds_kernel(const int64_t *__restrict__ off, int32_t V,
+                                     CsrExtremes *out) {
+    const int64_t want = threadIdx.x < 4 ? int64_t(1) << (16 >> threadIdx.x) : 2;
+    int64_t lo = 0, n = V;
+    while (n > 0) {
+        const int64_t h = n >> 1, v = lo + h;
+        const bool right = off[v + 1] - off[v] >= want;
+        lo = right ? v + 1 : lo;
+        n = right ? n - h - 1 : h;
+    }
+    out->below[threadIdx.x] = (int32_t)lo;
 }
 
 __global__ void hub_ids_kernel(int32_t n, int32_t V, int32_t *hubs, int32_t *slot) {
@@ -165,8 +179,10 @@ cudaError_t lower_offsets_device(const int64_t *off, const int32_t *adj, int32_t
 }
 
 cudaError_t csr_extremes_device(const int64_t *off, const int64_t *lo_off, int32_t V,
-                                int64_t light_below, CsrExtremes *out, cudaStream_t st) {
+                                int64_t light_below, bool ordered, CsrExtremes *out,
+                                cudaStream_t st) {
     extremes_init_kernel<<<1, 1, 0, st>>>(V, out);
+    if (ordered) degree_bounds_kernel<<<1, 5, 0, st>>>(off, V, out);
     extremes_kernel<<<V < (1 << 20) ? blocks_for(int64_t(V) + 1, 256) : 4096, 256, 0, st>>>(
         off, lo_off, V, light_below, out);
     return cudaGetLastError();
