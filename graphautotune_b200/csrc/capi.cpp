@@ -695,9 +695,10 @@ constexpr int64_t kRowMinDegree = 8;
 int upload_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes, bool ordered,
                 const HostGraph &h, cudaStream_t st) {
     if (min_degree <= 0 || max_bytes <= 0 || V == 0) return GAT_OK;
-    const int64_t words = (int64_t(V) + 31) / 32;
-    const int64_t fit = max_bytes / (words * 4);
-    const int64_t room = std::min(max_bytes, kSmallRowBytes) / (words * 4);
+    // rows hold whole 16-byte groups; the limits count a row's own words
+    const int64_t row_words = (int64_t(V) + 31) / 32, words = (row_words + 3) / 4 * 4;
+    const int64_t fit = max_bytes / (row_words * 4);
+    const int64_t room = std::min(max_bytes, kSmallRowBytes) / (row_words * 4);
     cudaError_t e;
     // Rows in decreasing order of degree: on the degree-ordered copy the
     // leading ids themselves, so only the counts are needed.

@@ -602,12 +602,10 @@ __device__ __forceinline__ int32_t min_level(const State &st, unsigned m) {
     return r;
 }
 
-// y equals one of the levels in `ex` (bit k stands for the lane's candidate).
+// y equals one of the levels in `m`.
 template <class State>
-__device__ __forceinline__ bool excluded(const State &st, unsigned ex, int k, int32_t cand,
-                                         int32_t y) {
-    bool r = ((ex >> k) & 1u) && y == cand;
-    unsigned m = ex & ~(1u << k);
+__device__ __forceinline__ bool excluded(const State &st, unsigned m, int32_t y) {
+    bool r = false;
     while (m) {
         const int j = __ffs(m) - 1;
         m &= m - 1;
@@ -641,130 +639,224 @@ __device__ __forceinline__ int32_t lane_cost(const State &st, const GatPlan &P, 
     return c;
 }
 
+// Bits of row[] at the elements of probe[0, n), one lane alone.  Eight row
+// words in flight: the lanes of a tile mostly probe the same list, so its
+// elements are broadcast reads and the row words are what takes time.
+__device__ __forceinline__ int probe_bits(const uint32_t *row, const int32_t *probe, int n) {
+    int c = 0, e = 0;
+    constexpr int kAhead = 8;
+    for (; e + kAhead <= n; e += kAhead) {
+        uint32_t w[kAhead];
+        int32_t y[kAhead];
+#pragma unroll
+        for (int t = 0; t < kAhead; t++) y[t] = probe[e + t];
+#pragma unroll
+        for (int t = 0; t < kAhead; t++) w[t] = __ldg(row + (y[t] >> 5));
+#pragma unroll
+        for (int t = 0; t < kAhead; t++) c += (w[t] >> (y[t] & 31)) & 1u;
+    }
+    for (; e < n; e++) {
+        const int32_t y = probe[e];
+        c += (__ldg(row + (y >> 5)) >> (y & 31)) & 1u;
+    }
+    return c;
+}
+
+// Common bits of two rows below T (rows are whole 16-byte groups).
+__device__ __forceinline__ int and_rows(const uint32_t *x, const uint32_t *y, int32_t T) {
+    int c = 0;
+    const int words = T >> 5, quads = words >> 2;
+    const uint4 *x4 = reinterpret_cast<const uint4 *>(x), *y4 = reinterpret_cast<const uint4 *>(y);
+#pragma unroll 2
+    for (int q = 0; q < quads; q++) {
+        const uint4 p = __ldg(x4 + q), r = __ldg(y4 + q);
+        c += __popc(p.x & r.x) + __popc(p.y & r.y) + __popc(p.z & r.z) + __popc(p.w & r.w);
+    }
+    for (int w = quads * 4; w < words; w++) c += __popc(__ldg(x + w) & __ldg(y + w));
+    if (T & 31) c += __popc(__ldg(x + words) & __ldg(y + words) & ((1u << (T & 31)) - 1u));
+    return c;
+}
+
+// The size |N(cand) n F| of one last-level set, by one lane alone, with the
+// bounds and exclusions of level_sets.  Both lists have rows: their words
+// below the bound are ANDed when that is less work than the probes (about 3.5
+// instructions a word against 6 an element).
+template <bool STATS, class State>
+__device__ __forceinline__ int lane_set(const State &st, const GatPlan &P, const SearchArgs &a,
+                                        int k, int p, int32_t cand, int i, const int32_t *nb,
+                                        int32_t dv, int hub_v, unsigned long long &by) {
+    const unsigned kbit = 1u << k;
+    const unsigned tm = P.p_trunc[p];
+    int32_t T = min_level(st, tm & ~kbit);
+    if (tm & kbit) T = min(T, cand);
+    if (P.p_kind[p] == GAT_SET_ALIAS) return cut_serial(a, cand, nb, dv, T);
+    const int f = P.p_father[p];
+    const int32_t *fp = st.set(f);
+    int32_t fl = st.len(P, f);
+    if (T != kInf) {
+        if (T == cand && f == P.l_loop[k])
+            fl = min(fl, i);
+        else if (tm != P.p_trunc[f])
+            fl = lower_serial(fp, fl, T);
+    }
+    const int owner_f = st.owner(f);
+    const int hub_f = (a.hub_slot != nullptr && owner_f >= 0) ? a.hub_slot[owner_f] : -1;
+    const uint32_t *row = nullptr;
+    const int32_t *probe = nullptr;
+    int np = 0;
+    int32_t nl = dv;
+    if (hub_v >= 0 && fl <= dv) {
+        row = a.bitmaps + (int64_t)hub_v * a.bitmap_words;
+        probe = fp;
+        np = fl;
+        if (STATS) nl = cut_serial(a, cand, nb, dv, T);
+    } else {
+        nl = cut_serial(a, cand, nb, dv, T);
+        const int shorter = min(nl, fl), longer = max(nl, fl);
+        const long long bs_cost = (long long)shorter * ceil_log2(longer + 1);
+        if (hub_v >= 0 && (long long)fl <= bs_cost && (hub_f < 0 || fl <= nl)) {
+            row = a.bitmaps + (int64_t)hub_v * a.bitmap_words;
+            probe = fp;
+            np = fl;
+        } else if (hub_f >= 0 && (long long)nl <= bs_cost) {
+            row = a.bitmaps + (int64_t)hub_f * a.bitmap_words;
+            probe = nb;
+            np = nl;
+        }
+    }
+    if (STATS) by += 4ull * (unsigned)(nl + fl);
+    // cand is never in N(cand), so its own exclusion holds by itself
+    unsigned m = P.p_excl[p] & ~kbit;
+    if (row) {
+        // An ALIAS father's list is its owner's row below the father's own
+        // bound, which is at least T.
+        const int32_t below = min(T, a.V);
+        int c;
+        if (hub_v >= 0 && hub_f >= 0 && (below >> 5) < 2 * np - (np >> 2)) {
+            const int32_t F = fl > 0 ? min(below, fp[fl - 1] + 1) : 0;
+            c = and_rows(a.bitmaps + (int64_t)hub_v * a.bitmap_words,
+                         a.bitmaps + (int64_t)hub_f * a.bitmap_words, F);
+        } else {
+            c = probe_bits(row, probe, np);
+        }
+        // an excluded vertex was counted if it is in both lists
+        while (m) {
+            const int32_t y = st.v(__ffs(m) - 1);
+            m &= m - 1;
+            if (bit_set(row, y) && contains(probe, np, y, 0)) c--;
+        }
+        return c;
+    }
+    const int32_t *sa = nl <= fl ? nb : fp;
+    const int32_t *lb = nl <= fl ? fp : nb;
+    const int ns = min(nl, fl), nlong = max(nl, fl);
+    const unsigned ex = m;
+    int c = 0;
+    if (nlong >= a.linear_below && merge_pays(ns, nlong)) {
+        merge_walk(sa, 0, ns, lb, nlong,
+                   [&](int32_t y) { c += excluded(st, ex, y) ? 0 : 1; });
+    } else {
+        for (int e = 0; e < ns; e++) {
+            const int32_t y = sa[e];
+            c += (contains(lb, nlong, y, a.linear_below) && !excluded(st, ex, y)) ? 1 : 0;
+        }
+    }
+    return c;
+}
+
+// Slot x's value: the size of its set, less the levels it must not count.
+template <class State>
+__device__ __forceinline__ long long lane_slot(const State &st, const GatPlan &P,
+                                               const SearchArgs &a, int k, int x, int32_t cand,
+                                               const int32_t *nb, int32_t here_len) {
+    const unsigned kbit = 1u << k;
+    const int p = P.iep_prefix[x];
+    const bool here = P.p_level[p] == k;
+    int32_t len = here ? here_len : st.len(P, p);
+    if (P.p_kind[p] == GAT_SET_COUNT) return len;
+    const int32_t *ptr = here ? nb : st.set(p);
+    const unsigned bm = P.iep_bound[x];
+    int32_t B = min_level(st, bm & ~kbit);
+    if (bm & kbit) B = min(B, cand);
+    if (B != kInf) len = lower_serial(ptr, len, B);
+    const unsigned m = P.iep_sub[x];
+    int h = 0;
+    for (int j = 0; j < P.basic; j++)
+        if ((m >> j) & 1u)
+            h += contains(ptr, len, j == k ? cand : st.v(j), a.linear_below) ? 1 : 0;
+    return (long long)len - h;
+}
+
 // The IEP value of one last-level candidate (level k = basic-1), formed by
 // one lane alone.  Every set of that level is either a count |N(cand) n F|
 // whose father F belongs to an earlier level or N(cand) itself, so nothing
 // has to be stored.  Each set and each IEP value is formed exactly as
-// level_sets and iep_value form it (same bounds, exclusions and
-// bitmap-or-search choice).  `i` is the candidate's position in its list.
+// level_sets and iep_value form it (same bounds, exclusions and choice of
+// lists).  `i` is the candidate's position in its list.  Up to kFewSets sets
+// and slots (all plans of five vertices and fewer but a few) stay in
+// registers; arrays indexed at run time live in local memory.
+constexpr int kFewSets = 3;
+
+template <class T>
+__device__ __forceinline__ T pick(int i, T x0, T x1, T x2) {
+    return i == 0 ? x0 : i == 1 ? x1 : x2;
+}
+
 template <bool STATS, class State>
 __device__ __forceinline__ unsigned long long lane_candidate(const State &st, const GatPlan &P,
                                                              const SearchArgs &a, int k,
                                                              int32_t cand, int i, bool hit,
                                                              unsigned long long &by) {
-    const unsigned kbit = 1u << k;
-    const int loop = P.l_loop[k];
     const int pb = P.l_pbegin[k], pe = P.l_pbegin[k + 1];
-    long long lv[8];   // level-k sets: count, or cut length of N(cand)
-    long long val[8];  // IEP slots
     const int64_t o = a.off[cand];
     const int32_t *nb = a.adj + o;
     const int32_t dv = (int32_t)(a.off[cand + 1] - o);
     const int hub_v = (a.hub_slot != nullptr) ? a.hub_slot[cand] : -1;
-    for (int p = pb; p < pe; p++) {
-        if (hit) {
-            lv[p - pb] = 0;
-            continue;
-        }
-        const unsigned tm = P.p_trunc[p];
-        int32_t T = min_level(st, tm & ~kbit);
-        if (tm & kbit) T = min(T, cand);
-        if (P.p_kind[p] == GAT_SET_ALIAS) {
-            lv[p - pb] = cut_serial(a, cand, nb, dv, T);
-            continue;
-        }
-        const int f = P.p_father[p];
-        const int32_t *fp = st.set(f);
-        int32_t fl = st.len(P, f);
-        if (T != kInf) {
-            if (T == cand && f == loop)
-                fl = min(fl, i);
-            else if (tm != P.p_trunc[f])
-                fl = lower_serial(fp, fl, T);
-        }
-        const int owner_f = st.owner(f);
-        const int hub_f = (a.hub_slot != nullptr && owner_f >= 0) ? a.hub_slot[owner_f] : -1;
-        const uint32_t *row = nullptr;
-        const int32_t *probe = nullptr;
-        int np = 0;
-        int32_t nl = dv;
-        if (hub_v >= 0 && fl <= dv) {
-            row = a.bitmaps + (int64_t)hub_v * a.bitmap_words;
-            probe = fp;
-            np = fl;
-            if (STATS) nl = cut_serial(a, cand, nb, dv, T);
-        } else {
-            nl = cut_serial(a, cand, nb, dv, T);
-            const int shorter = min(nl, fl), longer = max(nl, fl);
-            const long long bs_cost = (long long)shorter * ceil_log2(longer + 1);
-            if (hub_v >= 0 && (long long)fl <= bs_cost && (hub_f < 0 || fl <= nl)) {
-                row = a.bitmaps + (int64_t)hub_v * a.bitmap_words;
-                probe = fp;
-                np = fl;
-            } else if (hub_f >= 0 && (long long)nl <= bs_cost) {
-                row = a.bitmaps + (int64_t)hub_f * a.bitmap_words;
-                probe = nb;
-                np = nl;
-            }
-        }
-        if (STATS) by += 4ull * (unsigned)(nl + fl);
-        const unsigned ex = P.p_excl[p];
-        int c = 0;
-        if (row) {
-            for (int e = 0; e < np; e++) {
-                const int32_t y = probe[e];
-                c += (bit_set(row, y) && !excluded(st, ex, k, cand, y)) ? 1 : 0;
-            }
-        } else {
-            const int32_t *sa = nl <= fl ? nb : fp;
-            const int32_t *lb = nl <= fl ? fp : nb;
-            const int ns = min(nl, fl), nlong = max(nl, fl);
-            if (nlong >= a.linear_below && merge_pays(ns, nlong)) {
-                merge_walk(sa, 0, ns, lb, nlong, [&](int32_t y) {
-                    c += excluded(st, ex, k, cand, y) ? 0 : 1;
-                });
-            } else {
-                for (int e = 0; e < ns; e++) {
-                    const int32_t y = sa[e];
-                    c += (contains(lb, nlong, y, a.linear_below) &&
-                          !excluded(st, ex, k, cand, y))
-                             ? 1
-                             : 0;
-                }
-            }
-        }
-        lv[p - pb] = c;
-    }
-    for (int x = 0; x < P.iep_num; x++) {
-        const int p = P.iep_prefix[x];
-        const bool here = P.p_level[p] == k;
-        if (P.p_kind[p] == GAT_SET_COUNT) {
-            val[x] = here ? lv[p - pb] : (long long)st.len(P, p);
-            continue;
-        }
-        const int32_t *ptr = here ? nb : st.set(p);
-        int32_t len = here ? (int32_t)lv[p - pb] : st.len(P, p);
-        const unsigned bm = P.iep_bound[x];
-        int32_t B = min_level(st, bm & ~kbit);
-        if (bm & kbit) B = min(B, cand);
-        if (B != kInf) len = lower_serial(ptr, len, B);
-        const unsigned m = P.iep_sub[x];
-        int h = 0;
-        for (int j = 0; j < P.basic; j++)
-            if ((m >> j) & 1u)
-                h += contains(ptr, len, j == k ? cand : st.v(j), a.linear_below) ? 1 : 0;
-        val[x] = (long long)len - h;
-    }
     unsigned long long local = 0, cur = 1;
     int last = -1;
-    for (int g = 0; g < P.num_terms; g++) {
-        const unsigned long long v = (unsigned long long)val[P.t_slot[g]];
+    auto term = [&](int g, unsigned long long v) {
         cur = (g == last + 1) ? v : cur * v;
         if (P.t_close[g]) {
             last = g;
             local += cur * (unsigned long long)(long long)P.t_coef[g];
         }
+    };
+    if (pe - pb <= kFewSets && P.iep_num <= kFewSets) {
+        int32_t l0 = 0, l1 = 0, l2 = 0;  // level-k sets: count, or cut length of N(cand)
+        for (int p = pb; p < pe && !hit; p++) {
+            const int32_t c = lane_set<STATS>(st, P, a, k, p, cand, i, nb, dv, hub_v, by);
+            if (p == pb)
+                l0 = c;
+            else if (p == pb + 1)
+                l1 = c;
+            else
+                l2 = c;
+        }
+        long long v0 = 0, v1 = 0, v2 = 0;  // IEP slots
+        for (int x = 0; x < P.iep_num; x++) {
+            const int at = P.iep_prefix[x] - pb;
+            const long long v = lane_slot(st, P, a, k, x, cand, nb, pick(at, l0, l1, l2));
+            if (x == 0)
+                v0 = v;
+            else if (x == 1)
+                v1 = v;
+            else
+                v2 = v;
+        }
+        for (int g = 0; g < P.num_terms; g++)
+            term(g, (unsigned long long)pick((int)P.t_slot[g], v0, v1, v2));
+        return local;
     }
+    int32_t lv[8];
+    long long val[8];
+    for (int p = pb; p < pe; p++)
+        lv[p - pb] =
+            hit ? 0 : lane_set<STATS>(st, P, a, k, p, cand, i, nb, dv, hub_v, by);
+    for (int x = 0; x < P.iep_num; x++) {
+        const int at = P.iep_prefix[x] - pb;
+        val[x] = lane_slot(st, P, a, k, x, cand, nb, at >= 0 && at < pe - pb ? lv[at] : 0);
+    }
+    for (int g = 0; g < P.num_terms; g++) term(g, (unsigned long long)val[P.t_slot[g]]);
     return local;
 }
 

@@ -25,7 +25,7 @@ struct DevGraphView {
     // the vertices with hub_slot[v] >= 0 (null when none were built).
     const int32_t *hub_slot = nullptr;
     const uint32_t *bitmaps = nullptr;
-    int64_t bitmap_words = 0;  // words per row = ceil(V / 32)
+    int64_t bitmap_words = 0;  // words per row: ceil(V / 32), up to whole 16-byte groups
 };
 
 // Fills one V-bit row per hub (rows must be zeroed first).
