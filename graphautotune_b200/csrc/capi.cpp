@@ -50,11 +50,25 @@ struct gat_pattern {
 struct gat_schedule {
     int mode = 0;
     bool trivial = false;  // n <= 2: counted on the host
+    bool five_cycle = false;  // counted by cycles5.cu where the graph fits it
     Pattern pattern;
     RefSchedule ref;
     PlanInfo plan;
     std::string json;
 };
+
+namespace {
+// The 5-cycle, rooted at its largest vertex by its exact plan (every other
+// level below v0, one embedding per cycle): the plan path and cycles5.cu give
+// the same whole-graph total.
+bool is_five_cycle(const gat_schedule &s) {
+    const GatPlan &p = s.plan.plan;
+    if (s.mode != GAT_MODE_EXACT || p.n != 5 || p.divisor != 1) return false;
+    for (int i = 0; i < 5; i++)
+        if (__builtin_popcount(s.pattern.row[i]) != 2) return false;
+    return pattern_connected(s.pattern);
+}
+}  // namespace
 
 struct DevCopy {
     int64_t *off = nullptr;
@@ -280,6 +294,7 @@ int gat_schedule_build_variant(const gat_pattern *p, int mode, const gat_graph *
                     return fail(GAT_ERR_ARGUMENT, "schedule variant out of range");
                 return fail(GAT_ERR_PATTERN, err);
             }
+            s->five_cycle = is_five_cycle(*s);
             std::string perm, r;
             for (size_t i = 0; i < s->plan.perm.size(); i++)
                 perm += (i ? "," : "") + std::to_string(s->plan.perm[i]);
@@ -1154,6 +1169,42 @@ int run_clique(gat_executor *e, const DevGraphView &view, int64_t vb, int64_t ve
     return GAT_OK;
 }
 
+// The exact 5-cycle count of a whole graph (cycles5.cu); no scratch.
+int run_c5(gat_executor *e, const DevGraphView &view, cudaStream_t strm, uint64_t *count,
+           gat_stats *stats, std::chrono::steady_clock::time_point t0) {
+    int occ = 0;
+    cudaError_t ce = c5_blocks_per_sm(view, &occ);
+    if (ce != cudaSuccess) return cuda_fail(ce, "5-cycle occupancy");
+    if (occ <= 0) return fail(GAT_ERR_CUDA, "5-cycle kernel does not fit on the device");
+    const int grid = e->cfg.num_blocks > 0 ? std::min(e->cfg.num_blocks, e->sms * occ)
+                                           : (int)std::min<int64_t>(view.V, int64_t(e->sms) * occ);
+    cudaEventRecord(e->ev0, strm);
+    ce = launch_c5(view, e->sms, grid, e->ctr, nullptr, strm);
+    if (ce != cudaSuccess) return cuda_fail(ce, "5-cycle launch");
+    cudaEventRecord(e->ev1, strm);
+    if ((ce = cudaMemcpyAsync(e->host_ctr, e->ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost,
+                              strm)) != cudaSuccess ||
+        (ce = cudaStreamSynchronize(strm)) != cudaSuccess)
+        return cuda_fail(ce, "5-cycle count");
+    float ms = 0;
+    cudaEventElapsedTime(&ms, e->ev0, e->ev1);
+    const int64_t raw = (int64_t)(e->host_ctr->result + e->host_ctr->bytes / 2);
+    *count = (uint64_t)raw;
+    gat_stats st{};
+    st.kernel_ms = ms;
+    st.raw_sum = raw;
+    st.divisor = 1;
+    st.tasks = (uint64_t)view.lo_total;
+    st.grid = grid;
+    st.block = 256;
+    st.tile = 32;
+    st.launches = 2;
+    st.total_ms =
+        std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+    if (stats) *stats = st;
+    return GAT_OK;
+}
+
 int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *stream,
                uint64_t *count, gat_stats *stats, bool balg, int64_t root_begin = -1,
                int64_t root_end = -1, int shard = 0, int num_shards = 0) {
@@ -1280,6 +1331,9 @@ int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *strea
         }
         return run_c4(e, view, *dc, vb, ve, shape, strm, balg, count, stats, t0);
     }
+    // (instrumented counts, root ranges and shards follow the plan)
+    if (!balg && !ranged && s->five_cycle && e->cfg.special_kernels == 1 && c5_fits(view))
+        return run_c5(e, view, strm, count, stats, t0);
     int occ = blocks_per_sm(shape.tile, shape.block, balg);
     if (occ <= 0) return fail(GAT_ERR_CUDA, "kernel does not fit on the device");
     shape.grid = e->cfg.num_blocks > 0 ? e->cfg.num_blocks : e->sms * occ;
@@ -1416,6 +1470,17 @@ struct gat_batch {
     std::vector<int64_t> divisors;
     std::vector<int> modes;
     std::vector<int64_t> raw;
+    // Whole 5-cycle jobs run as launches of their own after the queue's.
+    struct FiveCycle {
+        DevGraphView view;
+        int grid;
+        size_t job;
+    };
+    std::vector<FiveCycle> five;
+    size_t queued = 0;  // jobs in the queue
+    int sms = 0;
+    DevCounters *d_five = nullptr;
+    cudaError_t enqueue();  // everything one run does, on `stream`
     void release_device() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
@@ -1427,6 +1492,9 @@ struct gat_batch {
         dev_free(d_cursor);
         dev_free(d_results);
         dev_free(d_scratch);
+        dev_free(d_five);
+        d_five = nullptr;
+        five.clear();
         cudaFreeHost(h_results);
         d_plans = nullptr;
         d_jobs = nullptr;
@@ -1445,6 +1513,25 @@ struct gat_batch {
         if (stream) cudaStreamDestroy(stream);
     }
 };
+
+cudaError_t gat_batch::enqueue() {
+    const size_t J = jobs.size();
+    cudaError_t e;
+    if ((e = cudaMemsetAsync(d_cursor, 0, sizeof(unsigned long long), stream)) != cudaSuccess ||
+        (e = cudaMemsetAsync(d_results, 0, sizeof(unsigned long long) * J, stream)) !=
+            cudaSuccess)
+        return e;
+    if (queued > 0 &&
+        (e = launch_batch(d_jobs, d_vstart, (int32_t)queued, vtotal, tile, grid, block, d_cursor,
+                          d_results, d_scratch, stride, stream)) != cudaSuccess)
+        return e;
+    for (size_t i = 0; i < five.size(); i++)
+        if ((e = launch_c5(five[i].view, sms, five[i].grid, d_five + i, d_results + five[i].job,
+                           stream)) != cudaSuccess)
+            return e;
+    return cudaMemcpyAsync(h_results, d_results, sizeof(unsigned long long) * J,
+                           cudaMemcpyDeviceToHost, stream);
+}
 
 extern "C" {
 
@@ -1534,8 +1621,12 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
         return fail(GAT_ERR_MEMORY, "batch plans");
     int64_t stride = 0;
     b->units = 0;
-    for (size_t q = 0; q < J; q++) {
-        const size_t j = order[q];
+    size_t q = 0;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    b->sms = sms;
+    for (size_t j : order) {
         gat_graph *g = b->jobs[j].g;
         const gat_schedule *s = b->jobs[j].s;
         const bool exact = s->mode == GAT_MODE_EXACT;
@@ -1548,9 +1639,22 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
         v.lo_off = dc.lo_off;
         v.lo_total = dc.lo_total;
         v.max_degree = dc.max_degree;
+        v.max_lower = dc.max_lower;
         v.hub_slot = dc.hub_slot;
         v.bitmaps = dc.bitmaps;
         v.bitmap_words = dc.bitmap_words;
+        b->divisors[j] = s->plan.plan.divisor;
+        b->modes[j] = s->mode;
+        if (s->five_cycle && b->jobs[j].num_shards == 0 && b->cfg.special_kernels == 1 &&
+            c5_fits(v)) {
+            int occ = 0;
+            if ((e = c5_blocks_per_sm(v, &occ)) != cudaSuccess) return cuda_fail(e, "5-cycle occupancy");
+            if (occ > 0) {
+                b->five.push_back({v, (int)std::min<int64_t>(v.V, int64_t(sms) * occ), j});
+                b->units += v.lo_total;
+                continue;
+            }
+        }
         plans[j] = s->plan.plan;
         if (b->cfg.special_kernels == 0) plans[j].lane_last = 0;
         batch_fill_job(host_jobs.data() + q * jb, b->d_plans + j, plans[j], v,
@@ -1558,15 +1662,12 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
                        b->jobs[j].shard, b->jobs[j].num_shards);
         stride = std::max<int64_t>(stride, tile_scratch_ints(plans[j], v.max_degree));
         b->units += batch_job_tasks(host_jobs.data() + q * jb);
-        b->divisors[j] = plans[j].divisor;
-        b->modes[j] = s->mode;
+        order[q++] = j;
     }
+    b->queued = q;
     b->stride = stride;
     int occ = batch_blocks_per_sm(b->tile, b->block);
     if (occ <= 0) return fail(GAT_ERR_CUDA, "batch kernel does not fit on the device");
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     b->grid = b->cfg.num_blocks > 0 ? b->cfg.num_blocks : sms * occ;
     const int64_t per_block = int64_t(b->block / b->tile) * stride * 4;
     const int64_t budget = b->cfg.memory_budget > 0 ? b->cfg.memory_budget : (int64_t(4) << 30);
@@ -1575,7 +1676,7 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
         b->grid = (int)std::min<int64_t>(b->grid, budget / per_block);
     }
     b->vtotal = 0;
-    for (size_t q = 0; q < J; q++) {
+    for (q = 0; q < b->queued; q++) {
         vstart[q] = b->vtotal;
         b->vtotal += batch_job_grabs(host_jobs.data() + q * jb, plans[order[q]],
                                      int64_t(b->grid) * (b->block / b->tile), b->tile, b->chunk);
@@ -1586,6 +1687,9 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
         (e = dev_alloc((void **)&b->d_cursor, sizeof(unsigned long long), b->stream)) != cudaSuccess ||
         (e = dev_alloc((void **)&b->d_results, sizeof(unsigned long long) * J, b->stream)) != cudaSuccess ||
         (e = dev_alloc((void **)&b->d_scratch, b->scratch_bytes, b->stream)) != cudaSuccess ||
+        (!b->five.empty() &&
+         (e = dev_alloc((void **)&b->d_five, sizeof(DevCounters) * b->five.size(), b->stream)) !=
+             cudaSuccess) ||
         (e = cudaMallocHost(&b->h_results, sizeof(unsigned long long) * J)) != cudaSuccess)
         return fail(GAT_ERR_MEMORY, std::string("batch tables: ") + cudaGetErrorString(e));
     if ((e = cudaMemcpyAsync(b->d_plans, plans.data(), sizeof(GatPlan) * J,
@@ -1601,13 +1705,7 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
         if ((e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal)) !=
             cudaSuccess)
             return cuda_fail(e, "begin capture");
-        cudaMemsetAsync(b->d_cursor, 0, sizeof(unsigned long long), b->stream);
-        cudaMemsetAsync(b->d_results, 0, sizeof(unsigned long long) * J, b->stream);
-        cudaError_t le = launch_batch(b->d_jobs, b->d_vstart, (int32_t)J, b->vtotal, b->tile,
-                                      b->grid, b->block, b->d_cursor, b->d_results,
-                                      b->d_scratch, b->stride, b->stream);
-        cudaMemcpyAsync(b->h_results, b->d_results, sizeof(unsigned long long) * J,
-                        cudaMemcpyDeviceToHost, b->stream);
+        const cudaError_t le = b->enqueue();
         e = cudaStreamEndCapture(b->stream, &b->graph);
         if (le != cudaSuccess) return cuda_fail(le, "batch launch (capture)");
         if (e != cudaSuccess) return cuda_fail(e, "end capture");
@@ -1625,18 +1723,7 @@ int gat_batch_run(gat_batch *b, gat_stats *stats) {
     const size_t J = b->jobs.size();
     cudaError_t e;
     cudaEventRecord(b->ev0, b->stream);
-    if (b->use_graph) {
-        e = cudaGraphLaunch(b->exec, b->stream);
-    } else {
-        cudaMemsetAsync(b->d_cursor, 0, sizeof(unsigned long long), b->stream);
-        cudaMemsetAsync(b->d_results, 0, sizeof(unsigned long long) * J, b->stream);
-        e = launch_batch(b->d_jobs, b->d_vstart, (int32_t)J, b->vtotal, b->tile, b->grid,
-                         b->block, b->d_cursor, b->d_results, b->d_scratch, b->stride,
-                         b->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(b->h_results, b->d_results, sizeof(unsigned long long) * J,
-                                cudaMemcpyDeviceToHost, b->stream);
-    }
+    e = b->use_graph ? cudaGraphLaunch(b->exec, b->stream) : b->enqueue();
     if (e != cudaSuccess) return cuda_fail(e, "batch launch");
     cudaEventRecord(b->ev1, b->stream);
     if ((e = cudaStreamSynchronize(b->stream)) != cudaSuccess) return cuda_fail(e, "batch run");
@@ -1659,7 +1746,7 @@ int gat_batch_run(gat_batch *b, gat_stats *stats) {
         st.grid = b->grid;
         st.block = b->block;
         st.tile = b->tile;
-        st.launches = 1;
+        st.launches = (b->queued > 0 ? 1 : 0) + 3 * (int)b->five.size();
         st.tasks = (uint64_t)b->units;
         st.scratch_bytes = (int64_t)b->scratch_bytes;
         *stats = st;

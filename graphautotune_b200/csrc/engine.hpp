@@ -151,6 +151,16 @@ int64_t clique_list_ints(int64_t lo_total);
 void clique_blocks_per_sm(int k, bool stats, int *warp_occ, int *cta_occ);
 cudaError_t launch_clique(const CliqueLaunch &launch, cudaStream_t st);
 
+// Exact 5-cycle count of a whole graph by path counts at each cycle's largest
+// vertex (cycles5.cu), for graphs whose 16-bit path counters fit in shared
+// memory.  ctr->result + ctr->bytes / 2 is the count; `result` (may be null)
+// receives it on the device.  c5_blocks_per_sm runs first (it sets the
+// kernel's shared-memory limit, which a stream capture may not).
+bool c5_fits(const DevGraphView &g);
+cudaError_t c5_blocks_per_sm(const DevGraphView &g, int *blocks);
+cudaError_t launch_c5(const DevGraphView &g, int sms, int grid, DevCounters *ctr,
+                      unsigned long long *result, cudaStream_t stream);
+
 // Graph construction on the device (gen.cu).  Both write off[V + 1] (caller
 // allocated) and allocate *adj with pad_ints ints past the E entries; E is
 // the number of directed entries of the symmetric, loop-free, deduplicated

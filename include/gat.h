@@ -137,7 +137,9 @@ typedef struct gat_config {
                                       0 = 4 GiB */
     int32_t special_kernels;       /* 1: patterns with a dedicated kernel use
                                       it (exact 4-cycle, exact 4- to
-                                      7-cliques) and plans use the
+                                      7-cliques, whole-graph exact 5-cycle
+                                      on graphs of up to about 98,000
+                                      vertices) and plans use the
                                       lane-per-candidate last level; 2: the
                                       lane path but no dedicated kernel;
                                       0: the plan interpreter alone */
@@ -294,7 +296,8 @@ int gat_executor_count_shard_balg(gat_executor *e, gat_graph *g,
  * No single reference counterpart: the reference runs one pm process per
  * (pattern, graph, config) (tuning/tuning/role/driver.py:88-132).  A batch
  * counts many (schedule, graph) jobs of uneven size in ONE persistent launch:
- * the jobs' level-1 work queues are split into grabs, concatenated (jobs of
+ * the jobs' level-1 work queues (5-cycle jobs with a dedicated
+ * kernel excepted: those follow as launches of the same run) are split into grabs, concatenated (jobs of
  * the most levels and longest rows first) and drained by one atomic cursor, so small jobs do not leave the GPU
  * idle.  gat_batch_prepare fixes the launch shape from `c`, uploads graphs
  * that are not resident yet, builds the job table and, with use_cuda_graph,
