@@ -878,15 +878,16 @@ __device__ __forceinline__ unsigned heavy_lanes(const Tile<G> &t, int32_t cost) 
 // of the tile takes candidates i, i+G, ... of the level's loop list
 // src[0, n) (lane_candidate).  No shared-memory writes, no syncs, and no idle
 // lanes when the lists are shorter than the tile.  Returns the sum of the
-// candidates' IEP values on every lane.
+// candidates' IEP values on every lane.  Of `parts` slices of the list, slice
+// `part` alone (whole groups of G candidates).
 template <int G, bool STATS>
 __device__ unsigned long long lane_last_level(const Tile<G> &t, const TileSmem &S,
                                               const GatPlan &P, const SearchArgs &a, int k,
                                               unsigned long long &bytes, const int32_t *src,
-                                              int n) {
+                                              int n, int part = 0, int parts = 1) {
     const TileState st{S};
     unsigned long long sum = 0, by = 0;
-    for (int i = t.lane; i < n; i += G) {
+    for (int i = part * G + t.lane; i < n; i += parts * G) {
         const int32_t cand = src[i];
         const bool hit = collides(st, P, k, cand);
         // Exact plans skip a colliding candidate; reference plans keep it
@@ -987,6 +988,8 @@ __device__ __forceinline__ bool lane_worth(const TileSmem &S, const GatPlan &P, 
     return cnt >= fmax;
 }
 
+// (`part` of `parts`: only every parts-th level-2 candidate of the units, or
+// group of G of them where the lanes take them.)
 // Runs the level-1 units [start, end) of one job: each unit (v0, v1) is the
 // start of a depth-first walk over levels 2 .. basic-1.  Lane 0 of the tile
 // accumulates the units' IEP values in `acc`.
@@ -997,7 +1000,8 @@ template <int G, bool STATS, bool ALL_ENTRIES>
 __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const GatPlan &P,
                                           const SearchArgs &a, int64_t start, int64_t end,
                                           int32_t *scratch, unsigned long long &acc,
-                                          unsigned long long &bytes) {
+                                          unsigned long long &bytes, int part = 0,
+                                          int parts = 1) {
     const int basic = P.basic;
     if (!ALL_ENTRIES && basic == 2 && P.lane_last) {
         run_pairs<G, STATS>(t, S, P, a, start, end, scratch, acc, bytes);
@@ -1030,9 +1034,14 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
         setup_level(t, S, P, 2);
         if (basic == 3 && P.lane_last && lane_worth<G>(S, P, 2, S.cnt[2])) {
             const unsigned long long r =
-                lane_last_level<G, STATS>(t, S, P, a, 2, bytes, S.src[2], S.cnt[2]);
+                lane_last_level<G, STATS>(t, S, P, a, 2, bytes, S.src[2], S.cnt[2], part,
+                                          parts);
             if (t.lane == 0) acc += r;
             continue;
+        }
+        if (parts > 1) {
+            if (t.lane == 0) S.pos[2] = part;
+            t.sync();
         }
         int k = 2;
         while (k >= 2) {
@@ -1040,7 +1049,8 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
                 k--;
                 continue;
             }
-            const int32_t cand = S.src[k][S.pos[k]];
+            const int at = S.pos[k];
+            const int32_t cand = S.src[k][at];
             bool hit = false;
             unsigned dm = P.l_distinct[k];
             while (dm) {
@@ -1049,14 +1059,14 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
                 hit |= (S.v[j] == cand);
             }
             t.sync();
-            if (t.lane == 0) S.pos[k]++;
+            if (t.lane == 0) S.pos[k] = at + (k == 2 ? parts : 1);
             if (hit && !P.collide_clear) {
                 t.sync();
                 continue;
             }
             if (t.lane == 0) S.v[k] = cand;
             t.sync();
-            level_sets<G, STATS>(t, S, P, a, k, cand, hit, scratch, bytes, S.pos[k] - 1);
+            level_sets<G, STATS>(t, S, P, a, k, cand, hit, scratch, bytes, at);
             if (k == basic - 1) {
                 const long long r = iep_value(t, S, P, a.linear_below);
                 if (t.lane == 0) acc += (unsigned long long)r;
@@ -1093,6 +1103,22 @@ __host__ __device__ __forceinline__ int64_t grab_units(int64_t left, int64_t til
     return c < unit ? unit : (c > most ? most : c);
 }
 
+// Parts a unit of four levels or more is split into, by its level-2
+// candidates.  With few units per tile the heaviest unit alone is the count's
+// time (6-cycle with chord on R-MAT 2^10, 12,016 units: 2.1 ms whole, 1.4 in
+// 6 parts).  A part forms the unit's first sets again, so units are split
+// only until there are 16 parts a tile, and not at all where a unit is one
+// level deep (house by the reference's rules on R-MAT 2^12: 1.39 ms whole,
+// 1.73 in 5 parts).
+constexpr int kSplitShare = 16;
+constexpr int kMostParts = 32;
+
+__host__ __device__ __forceinline__ int unit_parts(int64_t units, int64_t tiles, int basic) {
+    if (basic < 4 || units <= 0) return 1;
+    const int64_t p = tiles * kSplitShare / units;
+    return (int)(p < 1 ? 1 : p > kMostParts ? kMostParts : p);
+}
+
 template <int G, bool STATS, bool ALL_ENTRIES = false>
 __global__ void __launch_bounds__(256, 4)
     search_kernel(const SearchArgs a) {
@@ -1109,8 +1135,19 @@ __global__ void __launch_bounds__(256, 4)
     const bool pairs = !ALL_ENTRIES && P.basic == 2 && P.lane_last;
     const int64_t tiles = (int64_t)gridDim.x * tiles_per_block;
     int64_t left = a.num_tasks - a.task_begin;
+    // (a grab of a split queue is one part of one unit)
+    const int parts = unit_parts(left, tiles, P.basic);
     for (;;) {
         unsigned long long start = 0;
+        if (parts > 1) {
+            if (t.lane == 0) start = atomicAdd(&a.ctr->cursor, 1ull);
+            start = t.bcast(start, 0);
+            const int64_t unit = a.task_begin + (int64_t)(start / (unsigned)parts);
+            if (unit >= a.num_tasks) break;
+            run_units<G, STATS, ALL_ENTRIES>(t, S, P, a, unit, unit + 1, scratch, acc, bytes,
+                                             (int)(start % (unsigned)parts), parts);
+            continue;
+        }
         const int64_t take = grab_units(left, tiles, pairs, G, a.chunk);
         if (t.lane == 0)
             start = (unsigned long long)a.task_begin +

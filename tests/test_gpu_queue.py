@@ -48,3 +48,21 @@ def test_two_level_units_of_many_rows(gat, oracle, tile, block, chunk, blocks):
     b.prepare(c)
     b.run()
     assert b.counts() == want
+
+
+@pytest.mark.parametrize("tile,blocks", [(32, 0), (8, 0), (1, 0), (32, 1)])
+def test_units_split_into_parts(gat, oracle, tile, blocks):
+    """Plans of four levels and more on graphs with few units per tile (and,
+    with one CTA, many): candidates of level 2 dealt to the parts of a unit."""
+    c = gat.Config.engine_default()
+    c.threads_per_warp, c.num_blocks, c.special_kernels = tile, blocks, 2
+    ex = gat.Executor(c)
+    cycle6_chord = "010101101000010100101010000101100010"
+    for g in (gat.Graph.erdos_renyi(60, 7.0, 2), gat.Graph.barabasi_albert(90, 4, 3)):
+        off, adj = g.csr()
+        for p in ("0001100101010101010011000", "0111110111110111110111110", cycle6_chord):
+            s = gat.Schedule(p, "exact")
+            want = oracle.exact_count(off, adj, p)
+            assert ex.count(g, s).count == want, p
+            parts = [ex.count_shard(g, s, i, 3) for i in range(3)]
+            assert sum(r for r, _ in parts) == want * parts[0][1].divisor, p
