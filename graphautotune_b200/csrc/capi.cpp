@@ -146,6 +146,7 @@ struct gat_executor {
     int32_t *scratch = nullptr;
     size_t scratch_bytes = 0;
     bool scratch_clean = false;  // all-zero (the 4-cycle kernel's invariant)
+    int c4_light_occ[2] = {}, c4_root_occ[2][2] = {};  // CTAs per SM, 0: not asked yet
     DevCounters *ctr = nullptr;
     DevCounters *host_ctr = nullptr;  // pinned
     GatPlan *d_plan = nullptr;
@@ -1019,9 +1020,11 @@ namespace {
 int run_c4(gat_executor *e, const DevGraphView &view, const DevCopy &dc, int64_t vb,
            int64_t ve, LaunchShape shape, cudaStream_t strm, bool balg, uint64_t *count,
            gat_stats *stats, std::chrono::steady_clock::time_point t0) {
-    const int root_threads = c4_root_threads(view.E);
-    const int locc = c4_light_blocks_per_sm(balg);
-    const int rocc = c4_root_blocks_per_sm(root_threads, balg);
+    const int root_threads = c4_root_threads(view.E, dc.heavy_rows);
+    // (asked once per executor: the device does not change under it)
+    int &locc = e->c4_light_occ[balg], &rocc = e->c4_root_occ[balg][root_threads == 1024];
+    if (locc <= 0) locc = c4_light_blocks_per_sm(balg);
+    if (rocc <= 0) rocc = c4_root_blocks_per_sm(root_threads, balg);
     if (locc <= 0 || rocc <= 0) return fail(GAT_ERR_CUDA, "4-cycle kernels do not fit on the device");
     // Heavy roots: the leading run of ids with degree >= kC4HeavyDegree (on a
     // degree-ordered copy, exactly the vertices of that degree) take a CTA
@@ -1042,7 +1045,7 @@ int run_c4(gat_executor *e, const DevGraphView &view, const DevCopy &dc, int64_t
         cudaFree(e->scratch);
         e->scratch = nullptr;
         e->scratch_bytes = 0;
-        if ((ce = cudaMalloc(&e->scratch, need)) != cudaSuccess)
+        if ((ce = plain_alloc((void **)&e->scratch, need)) != cudaSuccess)
             return fail(GAT_ERR_MEMORY, std::string("4-cycle scratch: ") + cudaGetErrorString(ce));
         e->scratch_bytes = need;
     }
@@ -1118,7 +1121,7 @@ int run_clique(gat_executor *e, const DevGraphView &view, int64_t vb, int64_t ve
         cudaFree(e->scratch);
         e->scratch = nullptr;
         e->scratch_bytes = 0;
-        if ((ce = cudaMalloc(&e->scratch, need)) != cudaSuccess)
+        if ((ce = plain_alloc((void **)&e->scratch, need)) != cudaSuccess)
             return fail(GAT_ERR_MEMORY, std::string("clique scratch: ") + cudaGetErrorString(ce));
         e->scratch_bytes = need;
     }
@@ -1354,7 +1357,7 @@ int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *strea
         cudaFree(e->scratch);
         e->scratch = nullptr;
         e->scratch_bytes = 0;
-        if ((ce = cudaMalloc(&e->scratch, need)) != cudaSuccess)
+        if ((ce = plain_alloc((void **)&e->scratch, need)) != cudaSuccess)
             return fail(GAT_ERR_MEMORY, std::string("scratch allocation: ") + cudaGetErrorString(ce));
         e->scratch_bytes = need;
     }

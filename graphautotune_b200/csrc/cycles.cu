@@ -15,8 +15,8 @@
 //  * c4_light_kernel: a warp per root (roots of degree below the heavy
 //    threshold).  Lanes take the root's upper neighbours v1, find where
 //    N(v1) rises above v0 and add up the wedges W.  With W <= kWarpWedges
-//    the lanes walk their lists into a warp-private open-addressing table in
-//    shared memory (key x, count c), then read every slot once, add C(c, 2)
+//    the warp takes the lists end to end into an open-addressing table of
+//    its own in shared memory (key x, count c), then read every slot once, add C(c, 2)
 //    and clear it.  A root with more wedges is appended to a deferred list.
 //  * c4_root_kernel: a CTA per root, for the heavy roots and the deferred
 //    ones, largest degree first.  Segment starts (N(v1) above v0) are found
@@ -36,8 +36,9 @@
 // largest thousand.  R-MAT 2^20 (5.65e9 wedges) on a B200, ms per CTA: roots
 // of a million wedges and more 5.1 (76% of all wedges), others 3.3, reading
 // counters out 2, finding segments 1.3, tables 1.5; the light kernel 0.9.
-// One count: 21.4 ms with a search per entry and 16-bit windows, now 13.9;
-// R-MAT 2^18 3.2 -> 2.4, Barabasi-Albert 60,000 x 9 0.66 -> 0.26.
+// One count: 21.4 ms with a search per entry, 16-bit windows and a lane per
+// list in the light kernel, now 12.6; R-MAT 2^18 3.2 -> 2.15, Barabasi-Albert
+// 60,000 x 9 0.66 -> 0.23.
 //
 // Neither kernel waits on another CTA; the deferred list is written by the
 // first launch and read by the second, ordered on the stream.
@@ -52,7 +53,13 @@ namespace {
 
 constexpr int32_t kEmpty = 0;  // wedge endpoints lie above their root, so no key is 0
 constexpr int kWarpSlots = 1024;          // per-warp table slots
-constexpr int kWarpWedges = kWarpSlots / 2;
+constexpr int kWarpBits = 10;
+static_assert((1 << kWarpBits) == kWarpSlots, "table size is a power of two");
+// Most wedges of a warp's root: probes get long as the table fills (a warp
+// repeats one for its slowest lane), and a CTA costs about 3 us a root.  At
+// 1/4, 1/2 and 3/4 of the slots G(5,000, 20) took 76, 85 and 115 us a count,
+// G(30,000, 20) 201, 126 and 139, Barabasi-Albert 20,000 x 9 135, 141 and 212.
+constexpr int kWarpWedges = kWarpSlots * 3 / 8;
 constexpr int kLightBlock = 256;          // 8 warps
 // The root kernel in two shapes.  Two CTAs of 512 threads per SM hide one
 // root's barriers and chains of reads behind the other's (R-MAT 2^18: 2.2 ms
@@ -67,6 +74,7 @@ struct RootShape {
     static constexpr int kRegionBytes = 192 * BLOCK;        // counters or table
     static constexpr int kRegionWords = kRegionBytes / 4;
     static_assert(kSlots * 8 <= kRegionBytes, "table fits in the region");
+    static_assert((kSlots & (kSlots - 1)) == 0, "slots are a power of two");
 };
 
 __device__ __forceinline__ unsigned long long pairs_of(unsigned long long c) {
@@ -221,35 +229,74 @@ __global__ void __launch_bounds__(kLightBlock) c4_light_kernel(const LightArgs a
         const int32_t d0 = (int32_t)(a.off[v0 + 1] - o0);
         const int32_t lo0 = (int32_t)(a.lo_off[v0 + 1] - a.lo_off[v0]);
         if (d0 - lo0 < 2) continue;  // a cycle needs two neighbours above v0
-        // wedges of this root: sum over upper neighbours of |N(v1) above v0|
-        int32_t wl = 0;
-        for (int i = lo0 + lane; i < d0; i += 32) {
+        // This lane's upper neighbour of a group of 32: where its list rises
+        // above v0, and how many entries that leaves.
+        auto segment = [&](int i, int64_t &at) -> int32_t {
+            if (i >= d0) return 0;
             const int32_t v1 = a.adj[o0 + i];
             const int64_t o1 = a.off[v1];
             const int32_t d1 = (int32_t)(a.off[v1 + 1] - o1);
-            wl += d1 - above(a.adj + o1, a.lo_off, v1, (int32_t)v0);
+            const int32_t s1 = above(a.adj + o1, a.lo_off, v1, (int32_t)v0);
+            at = o1 + s1;
+            return d1 - s1;
+        };
+        // wedges of this root: sum over upper neighbours of |N(v1) above v0|
+        int32_t wl = 0, len = 0;
+        int64_t at = 0;
+        for (int i0 = lo0; i0 < d0; i0 += 32) {
+            len = segment(i0 + lane, at);
+            wl += len;
         }
-        int32_t W = wl;
-        for (int o = 16; o > 0; o >>= 1) W += __shfl_xor_sync(0xffffffffu, W, o);
+        const int32_t W = __reduce_add_sync(0xffffffffu, wl);
         if (W > kWarpWedges) {
             if (lane == 0) {
-                const unsigned long long at = atomicAdd(&a.aux->deferred_count, 1ull);
-                a.deferred[at] = (int32_t)v0;
+                const unsigned long long slot = atomicAdd(&a.aux->deferred_count, 1ull);
+                a.deferred[slot] = (int32_t)v0;
             }
             continue;
         }
         if (W < 2) continue;
-        for (int i = lo0 + lane; i < d0; i += 32) {
-            const int32_t v1 = a.adj[o0 + i];
-            const int64_t o1 = a.off[v1];
-            const int32_t d1 = (int32_t)(a.off[v1 + 1] - o1);
-            for (int32_t k = above(a.adj + o1, a.lo_off, v1, (int32_t)v0); k < d1; k++)
-                table_add(key, cnt, 10, a.adj[o1 + k], &a.ctr->error);
-            if (STATS) bytes += 20;
+        // A table of four slots a wedge and more where the warp's room has
+        // them: it is read out whole.
+        const int bits = min(kWarpBits, max(5, 32 - __clz(4 * W - 1)));
+        for (int i0 = lo0; i0 < d0; i0 += 32) {
+            if (d0 - lo0 > 32) len = segment(i0 + lane, at);  // else known from above
+            constexpr int kAhead = 4;
+            // The group's entries laid end to end, the lanes on consecutive
+            // ones: entry j belongs to the last lane whose exclusive prefix is
+            // at most j.  (A lane walking its own list takes as long as the
+            // longest: 34 us for 1,500 roots with a hub's list among theirs,
+            // 24 so; on a uniform G(30,000, 20) 146 us a count against 126.)
+            int32_t pre = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int32_t y = __shfl_up_sync(0xffffffffu, pre, o);
+                if (lane >= o) pre += y;
+            }
+            const int32_t total = __shfl_sync(0xffffffffu, pre, 31);
+            pre -= len;
+            for (int32_t j0 = 0; j0 < total; j0 += 32 * kAhead) {
+                int32_t xs[kAhead];
+#pragma unroll
+                for (int u = 0; u < kAhead; u++) {
+                    const int32_t j = j0 + 32 * u + lane;
+                    int own = 0;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1)
+                        if (__shfl_sync(0xffffffffu, pre, own + o) <= j) own += o;
+                    const int64_t from = __shfl_sync(0xffffffffu, at, own);
+                    const int32_t first = __shfl_sync(0xffffffffu, pre, own);
+                    xs[u] = j < total ? __ldg(a.adj + from + (j - first)) : 0;
+                }
+#pragma unroll
+                for (int u = 0; u < kAhead; u++)
+                    if (xs[u] > 0) table_add(key, cnt, bits, xs[u], &a.ctr->error);
+            }
+            if (STATS && i0 + lane < d0) bytes += 20;
         }
         if (STATS) bytes += 4ull * (unsigned)wl;
         __syncwarp();
-        for (int i = lane; i < kWarpSlots; i += 32) {
+        for (int i = lane; i < (1 << bits); i += 32) {
             if (key[i] != kEmpty) {
                 part += pairs_of(cnt[i]);
                 key[i] = kEmpty;
@@ -496,13 +543,20 @@ __device__ __forceinline__ unsigned long long drain_table(int32_t *key, uint32_t
     return part;
 }
 
-// Table bits for W wedges: at most half full.
+// Table bits for W wedges: at most an eighth full where the region has the
+// slots (a warp repeats a probe for its slowest lane), never over half.
+template <int BLOCK>
 __device__ __forceinline__ int table_bits(long long W) {
-    return max(8, 32 - __clz((int)(2 * W - 1)));
+    constexpr int kMost = 31 - __builtin_clz(RootShape<BLOCK>::kSlots);
+    return min(kMost, max(8, 32 - __clz((int)(8 * W - 1))));
 }
 
-// Graphs of fewer directed entries take the CTAs of 1,024 threads.
+// Graphs of fewer directed entries and at least this many heavy roots take
+// the CTAs of 1,024 threads (R-MAT 2^15: 193 us a count against 236;
+// Barabasi-Albert 20,000 x 9, 25 heavy roots and thousands of small ones, 164
+// against 142).
 constexpr int64_t kSmallEntries = 1 << 19;
+constexpr int64_t kFewHeavy = 64;
 
 // A CTA per root: heavy roots [heavy_begin, heavy_end) first, then the
 // deferred ones.  WIDE: 32-bit window counters (a count may reach 2^16).
@@ -517,11 +571,8 @@ __global__ void __launch_bounds__(BLOCK, RootShape<BLOCK>::kCtas)
     RootSmem<BLOCK> &S = *reinterpret_cast<RootSmem<BLOCK> *>(smem + kRegionBytes);
     int32_t *tkey = reinterpret_cast<int32_t *>(smem);
     uint32_t *tcnt = region + kCtaSlots;
-    // The region is all zero between roots: an empty table and cleared
-    // counters alike.
-    for (int i = threadIdx.x; i < kRegionWords; i += BLOCK) region[i] = 0u;
-    if (threadIdx.x == 0) S.next[0] = S.next[1] = 0;
     int parity = 0;
+    bool clear = false;  // the region has been cleared
     int32_t *cur = a.cursors + (int64_t)blockIdx.x * a.cursor_stride;
     const int64_t nheavy = a.heavy_end - a.heavy_begin;
     unsigned long long part = 0, bytes = 0;
@@ -541,6 +592,14 @@ __global__ void __launch_bounds__(BLOCK, RootShape<BLOCK>::kCtas)
         const int32_t lo0 = (int32_t)(a.lo_off[v0 + 1] - a.lo_off[v0]);
         const int32_t dp = d0 - lo0;
         if (dp < 2) continue;
+        if (!clear) {
+            // The region is all zero between roots: an empty table and
+            // cleared counters alike.  (A CTA that gets no root leaves it.)
+            for (int i = threadIdx.x; i < kRegionWords / 4; i += BLOCK)
+                reinterpret_cast<uint4 *>(region)[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (threadIdx.x == 0) S.next[0] = S.next[1] = 0;
+            clear = true;
+        }
         const int32_t *U = a.adj + o0 + lo0;
         const int ngroups = (dp + BLOCK - 1) / BLOCK;
         // Segment starts; one group's positions stay in registers, more go
@@ -602,7 +661,7 @@ __global__ void __launch_bounds__(BLOCK, RootShape<BLOCK>::kCtas)
         };
         // Everything from the cursors on through the CTA table.
         auto rest_by_table = [&](long long wedges) {
-            const int bits = table_bits(wedges);
+            const int bits = table_bits<BLOCK>(wedges);
             for (int g = 0; g < ngroups; g++) {
                 int64_t base = 0;
                 const int32_t len = take(g, a.V, base);
@@ -713,7 +772,9 @@ int c4_light_blocks_per_sm(bool stats) {
     return stats ? light_occupancy<true>() : light_occupancy<false>();
 }
 
-int c4_root_threads(int64_t E) { return E < kSmallEntries ? 1024 : 512; }
+int c4_root_threads(int64_t E, int64_t heavy_rows) {
+    return E < kSmallEntries && heavy_rows >= kFewHeavy ? 1024 : 512;
+}
 
 int c4_root_blocks_per_sm(int threads, bool stats) {
     if (threads == 1024)

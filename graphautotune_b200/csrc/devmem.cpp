@@ -54,6 +54,20 @@ cudaError_t pool_of(int dev, Pool **out) {
     return cudaSuccess;
 }
 
+// Gives back every pool's unused pages.
+void trim_locked() {
+    for (Pool &p : g_pools)
+        if (p.pool) {
+            cudaStreamSynchronize(p.frees);
+            cudaMemPoolTrimTo(p.pool, 0);
+        }
+}
+
+void trim_pools() {
+    std::lock_guard<std::mutex> lk(g_mu);
+    trim_locked();
+}
+
 }  // namespace
 
 cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t st) {
@@ -68,7 +82,20 @@ cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t st) {
         if ((e = pool_of(dev, &q)) != cudaSuccess) return e;
         pool = q->pool;
     }
+    e = cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, st);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();  // blocks of another size may hold the room
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
+    trim_pools();
     return cudaMallocFromPoolAsync(p, bytes ? bytes : 1, pool, st);
+}
+
+cudaError_t plain_alloc(void **p, size_t bytes) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    trim_pools();
+    return cudaMalloc(p, bytes);
 }
 
 cudaError_t dev_free(void *p, cudaStream_t st) { return p ? cudaFreeAsync(p, st) : cudaSuccess; }
@@ -97,12 +124,7 @@ PoolUser::PoolUser() {
 
 PoolUser::~PoolUser() {
     std::lock_guard<std::mutex> lk(g_mu);
-    if (--g_users > 0) return;
-    for (Pool &p : g_pools)
-        if (p.pool) {
-            cudaStreamSynchronize(p.frees);
-            cudaMemPoolTrimTo(p.pool, 0);
-        }
+    if (--g_users == 0) trim_locked();
 }
 
 }  // namespace gat

@@ -16,6 +16,10 @@ cudaError_t dev_alloc(void **p, size_t bytes, cudaStream_t st);
 cudaError_t dev_free(void *p, cudaStream_t st);
 void dev_free(void *p);
 
+// cudaMalloc, once more after the pools' unused pages are given back if the
+// device has no room (scratch that an executor keeps).
+cudaError_t plain_alloc(void **p, size_t bytes);
+
 // Counts the library's live handles (graphs, executors, batches).  The
 // pools keep up to kPoolKeepBytes for the next graph while there is one, and
 // give everything back when the last is freed.
