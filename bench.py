@@ -266,11 +266,16 @@ def naive_plan(off, adj, pattern: str, scans_per_stratum: int, seed: int = 12345
     return {"pattern": pattern, "units": units, "strata": strata}
 
 
+NAIVE = ROOT / "oracle/_ref/naive_sample"
+NO_NAIVE = ("oracle/_ref/naive_sample is not built (make -C oracle builds it where the "
+            "reference's sources are)")
+
+
 def run_naive(plan: dict, threads: int) -> dict:
     """Times the reference's naive matcher (oracle/_ref/naive_sample, built
     from target/naive_pm.cu) on the plan's units on `threads` threads, and
     per stratum (labelled embeddings, thread-seconds)."""
-    binary = ROOT / "oracle/_ref/naive_sample"
+    binary = NAIVE
     lines = "\n".join(f"{a} {b} {c}" for a, b, c in plan["units"]) + "\n"
     out = subprocess.run([str(binary), str(graph_cache_path()), plan["pattern"], "-",
                           str(threads)], input=lines, capture_output=True, text=True,
@@ -422,6 +427,9 @@ def exact_counts() -> dict | None:
 def run_reference(args):
     ws, rank, _ = dist_env()
     if rank != 0:
+        return 0
+    if not NAIVE.exists():
+        print(json.dumps({"impl": "reference", "unavailable": NO_NAIVE}), flush=True)
         return 0
     sys.path.insert(0, str(ROOT / "oracle"))
     import pyoracle
@@ -618,10 +626,16 @@ def cpu_baselines(off, adj, ex, gr, scheds) -> dict:
     sys.path.insert(0, str(ROOT / "oracle"))
     import pyoracle
 
-    auts = [pyoracle.automorphisms(p) for p in PATTERNS.values()]
-    plans = naive_plans(off, adj, 10.0, threads)
-    runs = [run_naive(pl, threads) for pl in plans]
-    est = naive_estimate(plans, runs, auts, threads)
+    naive = {"value": None, "kind": "reference", "sample": NO_NAIVE}
+    if NAIVE.exists():
+        auts = [pyoracle.automorphisms(p) for p in PATTERNS.values()]
+        plans = naive_plans(off, adj, 10.0, threads)
+        runs = [run_naive(pl, threads) for pl in plans]
+        est = naive_estimate(plans, runs, auts, threads)
+        naive = {"value": est["value"], "kind": "reference",
+                 "sample": naive_sample_text(plans, runs, threads),
+                 "matches_on_sample": est["matches_on_sample"],
+                 "estimated_workload_seconds": est["estimated_workload_seconds"]}
     port = oracle_port(off, adj, threads)
     gpu_ms, gpu_matches = 0.0, 0
     for name, rs in port.pop("ranges").items():
@@ -632,11 +646,7 @@ def cpu_baselines(off, adj, ex, gr, scheds) -> dict:
     assert gpu_matches == port["matches"], (gpu_matches, port["matches"])
     port["engine_on_same_ranges"] = {"value": gpu_matches / (gpu_ms / 1000.0),
                                      "unit": "matches/s", "device_ms": gpu_ms}
-    return {"value": est["value"], "unit": "matches/s", "cores": threads, "kind": "reference",
-            "sample": naive_sample_text(plans, runs, threads),
-            "matches_on_sample": est["matches_on_sample"],
-            "estimated_workload_seconds": est["estimated_workload_seconds"],
-            "oracle_port": port}
+    return {"unit": "matches/s", "cores": threads, **naive, "oracle_port": port}
 
 
 def run_profile_case(args):
