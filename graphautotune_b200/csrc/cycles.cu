@@ -14,7 +14,7 @@
 //
 //  * c4_light_kernel: a warp per root (roots of degree below the heavy
 //    threshold).  Lanes take the root's upper neighbours v1, find where
-//    N(v1) rises above v0 and add up the wedges W.  With W <= kWarpWedges
+//    N(v1) rises above v0 and add up the wedges W.  With few of them
 //    the warp takes the lists end to end into an open-addressing table of
 //    its own in shared memory (key x, count c), then read every slot once, add C(c, 2)
 //    and clear it.  A root with more wedges is appended to a deferred list.
@@ -59,7 +59,11 @@ static_assert((1 << kWarpBits) == kWarpSlots, "table size is a power of two");
 // repeats one for its slowest lane), and a CTA costs about 3 us a root.  At
 // 1/4, 1/2 and 3/4 of the slots G(5,000, 20) took 76, 85 and 115 us a count,
 // G(30,000, 20) 201, 126 and 139, Barabasi-Albert 20,000 x 9 135, 141 and 212.
-constexpr int kWarpWedges = kWarpSlots * 3 / 8;
+// Where the roots are few the CTAs have the time, so a quarter up to
+// kFewRoots vertices (G(5,000, 20) 76 us a count against 86, R-MAT 2^13 89
+// against 99) and three eighths beyond (G(30,000, 20) 153 against 201).
+constexpr int64_t kFewRoots = 8192;
+constexpr int warp_wedges(int64_t V) { return V <= kFewRoots ? kWarpSlots / 4 : kWarpSlots * 3 / 8; }
 constexpr int kLightBlock = 256;          // 8 warps
 // The root kernel in two shapes.  Two CTAs of 512 threads per SM hide one
 // root's barriers and chains of reads behind the other's (R-MAT 2^18: 2.2 ms
@@ -194,6 +198,7 @@ struct LightArgs {
     int32_t V;
     int32_t mark[kMarks];  // window ends (V: none), and where every row passes
     int32_t *marks;        // them: kMarks x V positions
+    int32_t most;          // wedges of a root that its warp counts itself
 };
 
 // A warp per root of [v_begin, v_end), roots handed out one at a time.
@@ -248,7 +253,7 @@ __global__ void __launch_bounds__(kLightBlock) c4_light_kernel(const LightArgs a
             wl += len;
         }
         const int32_t W = __reduce_add_sync(0xffffffffu, wl);
-        if (W > kWarpWedges) {
+        if (W > a.most) {
             if (lane == 0) {
                 const unsigned long long slot = atomicAdd(&a.aux->deferred_count, 1ull);
                 a.deferred[slot] = (int32_t)v0;
@@ -803,7 +808,8 @@ cudaError_t launch_c4(const C4Launch &L, cudaStream_t st) {
     const int64_t lb = std::max(L.v_begin, L.heavy_end), le = L.v_end;
     const bool roots = L.v_begin < L.v_end;
     if (lb < le || (roots && marked)) {
-        LightArgs la{g.off, g.adj, g.lo_off, lb, le, L.ctr, L.aux, L.deferred, g.V, {}, L.marks};
+        LightArgs la{g.off, g.adj, g.lo_off, lb, le, L.ctr, L.aux, L.deferred, g.V, {}, L.marks,
+                     warp_wedges(g.V)};
         for (int m = 0; m < kMarks; m++) la.mark[m] = mark[m];
         if ((e = L.stats ? light_attr<true>() : light_attr<false>()) != cudaSuccess) return e;
         if (L.stats)
