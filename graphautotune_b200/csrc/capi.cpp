@@ -708,8 +708,8 @@ void release_hubs(DevCopy &d) {
 constexpr int64_t kSmallRowBytes = int64_t(64) << 20;
 constexpr int64_t kRowMinDegree = 8;
 
-int upload_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes, bool ordered,
-                const HostGraph &h, cudaStream_t st) {
+int build_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes, bool ordered,
+               const HostGraph &h, cudaStream_t st) {
     if (min_degree <= 0 || max_bytes <= 0 || V == 0) return GAT_OK;
     // rows hold whole 16-byte groups; the limits count a row's own words
     const int64_t row_words = (int64_t(V) + 31) / 32, words = (row_words + 3) / 4 * 4;
@@ -765,6 +765,18 @@ int upload_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes, bo
     d.nhubs = (int32_t)nhubs;
     d.bitmap_words = words;
     return GAT_OK;
+}
+
+// A copy has all of its bitmap arrays or none: one whose bitmaps did not fit
+// stays usable without them.
+int upload_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes, bool ordered,
+                const HostGraph &h, cudaStream_t st) {
+    const int rc = build_hubs(d, V, min_degree, max_bytes, ordered, h, st);
+    if (rc != GAT_OK) {
+        cudaStreamSynchronize(st);  // part of them may be in the making
+        release_hubs(d);
+    }
+    return rc;
 }
 
 // Builds the given-id copy's hub bitmaps if the last upload deferred them.

@@ -975,7 +975,7 @@ cudaError_t launch_clique(const CliqueLaunch &L, cudaStream_t st) {
     if ((e = cudaMemsetAsync(L.ctr, 0, sizeof(DevCounters), st)) != cudaSuccess ||
         (e = cudaMemsetAsync(L.aux, 0, sizeof(CliqueAux), st)) != cudaSuccess)
         return e;
-    CliqueArgs a{g.off, g.adj, g.lo_off, g.hub_slot, g.bitmaps, g.bitmap_words,
+    CliqueArgs a{g.off, g.adj, g.lo_off, g.bitmaps ? g.hub_slot : nullptr, g.bitmaps, g.bitmap_words,
                  L.v_begin, L.v_end, L.u_begin, L.u_end, L.ctr, L.aux, L.rows, L.rows_stride,
                  L.lists, {}};
     for (int b = 1; b < kCliqueLists; b++)

@@ -273,7 +273,7 @@ cudaError_t launch_c5(const DevGraphView &g, int sms, int grid, DevCounters *ctr
                       unsigned long long *result, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(ctr, 0, sizeof(DevCounters), st);
     if (e != cudaSuccess) return e;
-    C5Args a{g.off, g.adj, g.lo_off, g.hub_slot, g.bitmaps, g.bitmap_words,
+    C5Args a{g.off, g.adj, g.lo_off, g.bitmaps ? g.hub_slot : nullptr, g.bitmaps, g.bitmap_words,
              g.V,   g.E,   ctr,      g.max_lower};
     const int64_t need = (g.E + kThreads - 1) / kThreads;
     if (need > 0)

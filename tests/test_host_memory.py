@@ -1,0 +1,75 @@
+"""The library's handling of device memory, on a CUDA runtime in host memory
+(fake_gpu): what a call leaves behind when an allocation is refused."""
+import gc
+
+import numpy as np
+import pytest
+
+import fake_gpu
+
+K4, C4 = "0111101111011110", "0101101001011010"
+C5 = "0001100101010101010011000"
+HOUSE = "0100110110010110110010100"
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    return fake_gpu.Fake(fake_gpu.build(tmp_path_factory.mktemp("fake")))
+
+
+@pytest.fixture
+def on_fake(gat, fake, monkeypatch):
+    """The package's classes on the fake runtime."""
+    from graphautotune_b200 import _lib
+
+    for name, (res, args) in _lib._SIGS.items():
+        fn = getattr(fake.lib, name)
+        fn.restype, fn.argtypes = res, args
+    gc.collect()
+    monkeypatch.setattr(_lib, "_lib", fake.lib)
+    for name in fake_gpu.SLOTS:
+        if name != "live":
+            fake[name] = fake_gpu.NEVER if name in ("refuse", "throw") else 0
+    yield fake
+    gc.collect()  # handles go where they came from
+
+
+def test_bitmaps_that_do_not_fit(gat, on_fake):
+    """The upload that cannot get its bitmaps says so and leaves no part of
+    them; counts that follow, single and batched, run without bitmaps."""
+    g = gat.Graph.barabasi_albert(2000, 4, 1)
+    g.upload()  # 64 KB of neighbours, 8 KB a table of vertices
+    ex = gat.Executor()
+    for p in (K4, C4, HOUSE, C5):  # (the executor keeps the scratch of these)
+        ex.count(g, gat.Schedule(p, "exact"))
+    assert on_fake["c5_bitmaps"] == 1
+    g.upload(hub_min_degree=0)
+    live = on_fake["live"]
+    on_fake["refuse"] = 100_000
+    for degree_order in (True, False):
+        with pytest.raises(gat.GatError, match="GAT_ERR_MEMORY"):
+            g.upload(degree_order=degree_order)
+        if degree_order:
+            assert on_fake["live"] == live
+        for p in (C5, K4, C4, HOUSE):
+            ex.count(g, gat.Schedule(p, "exact"))
+        assert on_fake["c5_bitmaps"] == 0
+    # the copy with the given ids makes its bitmaps when a count asks for them
+    g.upload(hub_min_degree=0)
+    with pytest.raises(gat.GatError, match="GAT_ERR_MEMORY"):
+        g.upload()
+    ref = gat.Schedule(HOUSE, "ref")
+    with pytest.raises(gat.GatError, match="GAT_ERR_MEMORY"):
+        ex.count(g, ref)
+    ex.count(g, ref)
+    on_fake["refuse"] = fake_gpu.NEVER  # (a batch has scratch of its own)
+    b = gat.Batch()
+    for p in (C5, HOUSE):
+        b.add(g, gat.Schedule(p, "exact"))
+    b.prepare(cuda_graph=False)
+    b.run()
+    assert on_fake["c5_bitmaps"] == 0
+    g.upload()
+    ex.count(g, gat.Schedule(C5, "exact"))
+    assert on_fake["c5_bitmaps"] == 1
+    assert on_fake["misuse"] == 0
