@@ -58,10 +58,14 @@ struct Shape {
 };
 
 // A training step's two launches follow one another within a microsecond:
-// each may start while the other ends and waits here for its results.
+// each may start while the other ends and waits here for its results.  The
+// next launch is let in only after the wait, so that at most two overlap, and
+// what one launch writes and the next reads (parameters, activations, deltas)
+// is read past L1 (__ldcg): the read-only path may hold lines from before the
+// writer ran.
 __device__ __forceinline__ void after_previous_launch() {
-    cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
+    cudaTriggerProgrammaticLaunchCompletion();
 }
 
 constexpr int kW2Pitch = kHidden + 1;  // padded rows: lanes on k or on u, no conflicts
@@ -73,7 +77,7 @@ constexpr int kW2Pitch = kHidden + 1;  // padded rows: lanes on k or on u, no co
 //   dy_r = 2 (y_r - t_r) / n,  d2 = dy w3 . [h2 > 0],  d1 = (d2 W2^T) . [h1 > 0]
 template <bool BACK>
 __global__ void __launch_bounds__(256)
-    mlp_rows_kernel(const float *__restrict__ params, int in, const float *__restrict__ X,
+    mlp_rows_kernel(const float *params, int in, const float *__restrict__ X,
                     const int *__restrict__ order, const float *__restrict__ T, int n,
                     float *__restrict__ y, float *__restrict__ h1, float *__restrict__ h2,
                     float *__restrict__ dyo, float *__restrict__ d2o, float *__restrict__ d1o) {
@@ -88,14 +92,14 @@ __global__ void __launch_bounds__(256)
     const int q1 = (nw1 + kHidden) / 4, q2 = kHidden * kHidden / 4;
 #pragma unroll 4
     for (int i = threadIdx.x; i < q2; i += 256) {
-        const float4 v = p4[q1 + i];
+        const float4 v = __ldcg(p4 + q1 + i);
         float *to = W2 + (4 * i / kHidden) * kW2Pitch + 4 * i % kHidden;
         to[0] = v.x, to[1] = v.y, to[2] = v.z, to[3] = v.w;
     }
 #pragma unroll 4
-    for (int i = threadIdx.x; i < q1; i += 256) reinterpret_cast<float4 *>(sm)[i] = p4[i];
+    for (int i = threadIdx.x; i < q1; i += 256) reinterpret_cast<float4 *>(sm)[i] = __ldcg(p4 + i);
     for (int i = threadIdx.x; i < 2 * kHidden + 1; i += 256)
-        B2[i] = params[nw1 + kHidden + kHidden * kHidden + i];
+        B2[i] = __ldcg(params + nw1 + kHidden + kHidden * kHidden + i);
     __syncthreads();
     const float b3 = W3[kHidden];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -182,10 +186,8 @@ constexpr int kGradThreads = kGradRows * kHidden;
 template <bool ADAM>
 __global__ void __launch_bounds__(kGradThreads)
     mlp_param_kernel(int in, const float *__restrict__ X, const int *__restrict__ order,
-                     const float *__restrict__ h1, const float *__restrict__ h2,
-                     const float *__restrict__ dy, const float *__restrict__ d2,
-                     const float *__restrict__ d1, int n, float *__restrict__ grad,
-                     const AdamState adam) {
+                     const float *h1, const float *h2, const float *dy, const float *d2,
+                     const float *d1, int n, float *__restrict__ grad, const AdamState adam) {
     extern __shared__ float sm[];
     float *B = sm;                     // d1, d2 or h2 of the chunk's rows
     float *A = B + kChunk * kHidden;   // their factors
@@ -223,16 +225,16 @@ __global__ void __launch_bounds__(kGradThreads)
         const float4 *from = reinterpret_cast<const float4 *>(src + (int64_t)r0 * kHidden);
         float4 *to = reinterpret_cast<float4 *>(B);
 #pragma unroll 16
-        for (int i = threadIdx.x; i < rows * kHidden / 4; i += kGradThreads) to[i] = from[i];
+        for (int i = threadIdx.x; i < rows * kHidden / 4; i += kGradThreads) to[i] = __ldcg(from + i);
         for (int i = threadIdx.x; i < rows * kGradRows; i += kGradThreads) {
             const int r = r0 + i / kGradRows, c = row + i % kGradRows;
             float v = 0.f;
             if (kind == 0) {
                 if (c < in) v = X[(int64_t)(order ? order[r] : r) * in + c];
             } else if (kind == 1) {
-                v = h1[(int64_t)r * kHidden + c];
+                v = __ldcg(h1 + (int64_t)r * kHidden + c);
             } else if (kind == 4 && i % kGradRows == 0) {
-                v = dy[r];
+                v = __ldcg(dy + r);
             }
             A[i] = v;
         }
