@@ -249,15 +249,34 @@ size_t root_smem(const DevGraphView &g) {
 }  // namespace
 
 // Graphs that the path counts take: the counters fit in shared memory, and
-// the scan of V counters per root is no more than the plan's walk.  Measured
-// (path / plan, ms), G(n, d): 4,000 x 6 0.036 / 0.105, 32,000 x 7 0.51 / 0.80,
-// 64,000 x 7 3.4 / 1.8, 64,000 x 24 7.8 / 50, 95,000 x 20 12 / 48;
-// Barabasi-Albert 20,011 x 9 0.8 / 11.7, 60,000 x 4 4.8 / 5.4; R-MAT 2^13
-// 0.34 / 20: only graphs that are both sparse and large keep the plan.
+// scanning V counters per root is no more than the plan's walk.  The scan does
+// not fall with the density, the walk does: with 2 entries a vertex G(40,000)
+// takes 0.51 ms by paths and 0.10 by the plan.  Measured (path / plan, ms; d
+// entries a vertex):
+//   G(n, d)            d = 2          4           8            12
+//     n = 4,000     .027 / .074  .031 / .10   .037 / .22   .045 / .51
+//        16,000     .085 / .089  .12 / .19    .15 / .60    .18 / 1.6
+//        24,000     .16 / .10    .21 / .23    .29 / .87    .36 / 2.4
+//        40,000     .51 / .10    .74 / .36    1.0 / 1.5    1.3 / 4.1
+//        64,000     1.9 / .15    2.7 / .57    3.7 / 2.6    4.7 / 7.2
+//        95,000     3.5 / .22    5.0 / .82    6.6 / 4.0    8.3 / 11
+//   Barabasi-Albert 40,000  .77 / .53    1.0 / 1.6    1.5 / 4.0    2.1 / 8.2
+//                   64,000  2.8 / .76    3.6 / 2.3    5.4 / 5.9    7.3 / 13
+//   R-MAT of 2^15, 2^16 vertices, d = 2: .41 / 2.3, 2.5 / 6.2
+// Up to 2^14 vertices, and from 12 entries a vertex on, the paths were ahead on
+// every graph tried.  In between, a walk grows with the density and the longest
+// rows and lower lists, the scan with V^2 over the CTAs an SM holds; of 260
+// graphs of 12,000 to 95,000 vertices the line below sends none to the paths
+// that lose more than 1.37 times there, and none to the plan that lose more
+// than 1.56 (both a tenth of a ms to a few ms long).
 bool c5_fits(const DevGraphView &g) {
-    if (g.V <= 0 || g.lo_off == nullptr || g.max_lower >= 65536 || root_smem(g) > 200 * 1024)
-        return false;
-    return g.V <= 40000 || g.E >= int64_t(12) * g.V;
+    constexpr size_t kSmBytes = 227 * 1024, kCtaBytes = 1024;  // CTA: reserved by the system
+    const size_t smem = root_smem(g);
+    if (g.V <= 0 || g.lo_off == nullptr || g.max_lower >= 65536 || smem > 200 * 1024) return false;
+    if (g.V <= 16384 || g.E >= int64_t(12) * g.V) return true;
+    const double v = g.V, d = double(g.E) / v, lower = g.max_lower;
+    const double ctas = double(std::min<size_t>(2048 / kThreads, kSmBytes / (smem + kCtaBytes)));
+    return d * d * d * lower * lower * g.max_degree * ctas * ctas >= 2.5e-13 * v * v * v * v;
 }
 
 cudaError_t c5_blocks_per_sm(const DevGraphView &g, int *blocks) {

@@ -139,7 +139,8 @@ typedef struct gat_config {
                                       it (exact 4-cycle, exact 4- to
                                       7-cliques, whole-graph exact 5-cycle
                                       on graphs of up to about 98,000
-                                      vertices) and plans use the
+                                      vertices, sparse ones to 16,384)
+                                      and plans use the
                                       lane-per-candidate last level; 2: the
                                       lane path but no dedicated kernel;
                                       0: the plan interpreter alone */
