@@ -1184,6 +1184,12 @@ int run_clique(gat_executor *e, const DevGraphView &view, int64_t vb, int64_t ve
     return GAT_OK;
 }
 
+// CTAs of a 5-cycle count: the configured number, at most what is resident.
+int c5_grid(const gat_config &c, const DevGraphView &view, int sms, int occ) {
+    const int64_t want = c.num_blocks > 0 ? c.num_blocks : view.V;
+    return (int)std::min<int64_t>(want, int64_t(sms) * occ);
+}
+
 // The exact 5-cycle count of a whole graph (cycles5.cu); no scratch.
 int run_c5(gat_executor *e, const DevGraphView &view, cudaStream_t strm, uint64_t *count,
            gat_stats *stats, std::chrono::steady_clock::time_point t0) {
@@ -1191,8 +1197,7 @@ int run_c5(gat_executor *e, const DevGraphView &view, cudaStream_t strm, uint64_
     cudaError_t ce = c5_blocks_per_sm(view, &occ);
     if (ce != cudaSuccess) return cuda_fail(ce, "5-cycle occupancy");
     if (occ <= 0) return fail(GAT_ERR_CUDA, "5-cycle kernel does not fit on the device");
-    const int grid = e->cfg.num_blocks > 0 ? std::min(e->cfg.num_blocks, e->sms * occ)
-                                           : (int)std::min<int64_t>(view.V, int64_t(e->sms) * occ);
+    const int grid = c5_grid(e->cfg, view, e->sms, occ);
     cudaEventRecord(e->ev0, strm);
     ce = launch_c5(view, e->sms, grid, e->ctr, nullptr, strm);
     if (ce != cudaSuccess) return cuda_fail(ce, "5-cycle launch");
@@ -1665,7 +1670,7 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
             int occ = 0;
             if ((e = c5_blocks_per_sm(v, &occ)) != cudaSuccess) return cuda_fail(e, "5-cycle occupancy");
             if (occ > 0) {
-                b->five.push_back({v, (int)std::min<int64_t>(v.V, int64_t(sms) * occ), j});
+                b->five.push_back({v, c5_grid(b->cfg, v, sms, occ), j});
                 b->units += v.lo_total;
                 continue;
             }

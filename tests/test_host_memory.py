@@ -73,3 +73,24 @@ def test_bitmaps_that_do_not_fit(gat, on_fake):
     ex.count(g, gat.Schedule(C5, "exact"))
     assert on_fake["c5_bitmaps"] == 1
     assert on_fake["misuse"] == 0
+
+
+def _counted(gat, g, cfg):
+    """One count and one batch of the 5-cycle under a configuration."""
+    s = gat.Schedule(C5, "exact")
+    gat.Executor(cfg).count(g, s)
+    yield "count"
+    b = gat.Batch()
+    b.add(g, s)
+    b.prepare(cfg, cuda_graph=False)
+    b.run()
+    yield "batch"
+
+
+def test_five_cycles_take_num_blocks(gat, on_fake):
+    g = gat.Graph.barabasi_albert(500, 4, 1)
+    cfg = gat.Config.engine_default()
+    for blocks, grid in ((7, 7), (0, 200), (10_000, 200)):  # 100 SMs of two CTAs
+        cfg.num_blocks = blocks
+        for how in _counted(gat, g, cfg):
+            assert on_fake["c5_grid"] == grid, how
