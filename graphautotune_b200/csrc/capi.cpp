@@ -1184,6 +1184,15 @@ int run_clique(gat_executor *e, const DevGraphView &view, int64_t vb, int64_t ve
     return GAT_OK;
 }
 
+// The graph as a 5-cycle count under this configuration sees it.
+DevGraphView c5_view(const gat_config &c, DevGraphView view) {
+    if (c.hub_bitmaps == 0) {
+        view.hub_slot = nullptr;
+        view.bitmaps = nullptr;
+    }
+    return view;
+}
+
 // CTAs of a 5-cycle count: the configured number, at most what is resident.
 int c5_grid(const gat_config &c, const DevGraphView &view, int sms, int occ) {
     const int64_t want = c.num_blocks > 0 ? c.num_blocks : view.V;
@@ -1353,7 +1362,7 @@ int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *strea
     }
     // (instrumented counts, root ranges and shards follow the plan)
     if (!balg && !ranged && s->five_cycle && e->cfg.special_kernels == 1 && c5_fits(view))
-        return run_c5(e, view, strm, count, stats, t0);
+        return run_c5(e, c5_view(e->cfg, view), strm, count, stats, t0);
     int occ = blocks_per_sm(shape.tile, shape.block, balg);
     if (occ <= 0) return fail(GAT_ERR_CUDA, "kernel does not fit on the device");
     shape.grid = e->cfg.num_blocks > 0 ? e->cfg.num_blocks : e->sms * occ;
@@ -1670,7 +1679,7 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
             int occ = 0;
             if ((e = c5_blocks_per_sm(v, &occ)) != cudaSuccess) return cuda_fail(e, "5-cycle occupancy");
             if (occ > 0) {
-                b->five.push_back({v, c5_grid(b->cfg, v, sms, occ), j});
+                b->five.push_back({c5_view(b->cfg, v), c5_grid(b->cfg, v, sms, occ), j});
                 b->units += v.lo_total;
                 continue;
             }

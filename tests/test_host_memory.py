@@ -94,3 +94,13 @@ def test_five_cycles_take_num_blocks(gat, on_fake):
         cfg.num_blocks = blocks
         for how in _counted(gat, g, cfg):
             assert on_fake["c5_grid"] == grid, how
+
+
+def test_five_cycles_without_bitmaps(gat, on_fake):
+    """hub_bitmaps = 0: never, where the graph has them."""
+    g = gat.Graph.barabasi_albert(500, 4, 1)
+    cfg = gat.Config.engine_default()
+    for flag in (1, 0):
+        cfg.hub_bitmaps = flag
+        for how in _counted(gat, g, cfg):
+            assert on_fake["c5_bitmaps"] == flag, how
