@@ -70,6 +70,16 @@ bool is_five_cycle(const gat_schedule &s) {
 }
 }  // namespace
 
+// Device arrays that a graph has let go of, freed with the last holder: a
+// prepared batch and a count in flight hold the arrays they read, so that a
+// graph may be uploaded again, or freed, meanwhile.
+struct DevArrays {
+    void *p[3] = {};
+    ~DevArrays() {
+        for (void *q : p) dev_free(q);
+    }
+};
+
 struct DevCopy {
     int64_t *off = nullptr;
     int32_t *adj = nullptr;
@@ -90,18 +100,26 @@ struct DevCopy {
     uint32_t *bitmaps = nullptr;
     int32_t nhubs = 0;
     int64_t bitmap_words = 0;
-    void release() {
-        dev_free(off);
-        dev_free(adj);
-        dev_free(lo_off);
-        dev_free(hub_slot);
-        dev_free(hubs);
-        dev_free(bitmaps);
+    // Holders of (off, adj, lo_off) and of (hub_slot, hubs, bitmaps).
+    std::shared_ptr<DevArrays> rows = std::make_shared<DevArrays>(),
+                               hub_rows = std::make_shared<DevArrays>();
+    void release_hubs() {
+        hub_rows->p[0] = hub_slot;
+        hub_rows->p[1] = hubs;
+        hub_rows->p[2] = bitmaps;
+        hub_rows = std::make_shared<DevArrays>();
         hub_slot = nullptr;
         hubs = nullptr;
         bitmaps = nullptr;
         nhubs = 0;
         bitmap_words = 0;
+    }
+    void release() {
+        release_hubs();
+        rows->p[0] = off;
+        rows->p[1] = adj;
+        rows->p[2] = lo_off;
+        rows = std::make_shared<DevArrays>();
         off = nullptr;
         adj = nullptr;
         lo_off = nullptr;
@@ -684,17 +702,6 @@ int derive_ordered_copy(const HostGraph &h, const DevCopy &src, DevCopy &d, cuda
     return finish_copy(d, h.V, true, st);
 }
 
-void release_hubs(DevCopy &d) {
-    dev_free(d.hub_slot);
-    dev_free(d.hubs);
-    dev_free(d.bitmaps);
-    d.hub_slot = nullptr;
-    d.hubs = nullptr;
-    d.bitmaps = nullptr;
-    d.nhubs = 0;
-    d.bitmap_words = 0;
-}
-
 // Bitmap rows: the hubs (degree >= min_degree, largest degree first, as many
 // as fit in max_bytes), and below them further rows in degree order while all
 // rows together stay within kSmallRowBytes.  A set operation through a row
@@ -774,7 +781,7 @@ int upload_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes, bo
     const int rc = build_hubs(d, V, min_degree, max_bytes, ordered, h, st);
     if (rc != GAT_OK) {
         cudaStreamSynchronize(st);  // part of them may be in the making
-        release_hubs(d);
+        d.release_hubs();
     }
     return rc;
 }
@@ -927,7 +934,7 @@ int gat_graph_upload_ex(gat_graph *g, int flags, int64_t hub_min_degree,
     // is kept; its hub bitmaps are rebuilt for the requested parameters.
     int rc = GAT_OK;
     if (g->dev.ready && g->device == dev)
-        release_hubs(g->dev);
+        g->dev.release_hubs();
     else if ((rc = ensure_host_adj(g)) == GAT_OK)
         rc = upload_copy(g->host, g->dev, false, st);
     g->hub_min_degree = hub_min_degree;
@@ -938,7 +945,7 @@ int gat_graph_upload_ex(gat_graph *g, int flags, int64_t hub_min_degree,
     if (rc != GAT_OK) return rc;
     if (flags & GAT_UPLOAD_DEGREE_ORDER) {
         if (g->dev_ordered.ready && g->device == dev) {
-            release_hubs(g->dev_ordered);
+            g->dev_ordered.release_hubs();
             rc = GAT_OK;
         } else {
             // graphs too large for the device relabel are relabelled on the host
@@ -1269,6 +1276,7 @@ int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *strea
         if (rc != GAT_OK) return rc;
         dc = &g->dev;
     }
+    const std::shared_ptr<DevArrays> held[2] = {dc->rows, dc->hub_rows};
     DevGraphView view;
     view.V = g->host.V;
     view.E = g->host.E;
@@ -1496,6 +1504,7 @@ struct gat_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    std::vector<std::shared_ptr<DevArrays>> held;  // the jobs' graph arrays
     std::vector<int64_t> divisors;
     std::vector<int> modes;
     std::vector<int64_t> raw;
@@ -1524,6 +1533,7 @@ struct gat_batch {
         dev_free(d_five);
         d_five = nullptr;
         five.clear();
+        held.clear();
         cudaFreeHost(h_results);
         d_plans = nullptr;
         d_jobs = nullptr;
@@ -1660,6 +1670,8 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
         const gat_schedule *s = b->jobs[j].s;
         const bool exact = s->mode == GAT_MODE_EXACT;
         const DevCopy &dc = (exact && g->dev_ordered.ready) ? g->dev_ordered : g->dev;
+        b->held.push_back(dc.rows);
+        b->held.push_back(dc.hub_rows);
         DevGraphView v;
         v.V = g->host.V;
         v.E = g->host.E;

@@ -38,6 +38,12 @@ class Fake:
         self.lib = C.CDLL(str(path))
         self._state = (C.c_int64 * len(SLOTS)).in_dll(self.lib, "fake_state")
 
+    def during(self, call) -> None:
+        """call() runs while each counting kernel does (None: nothing)."""
+        self._during = C.CFUNCTYPE(None)(call) if call else None
+        C.c_void_p.in_dll(self.lib, "fake_during").value = (
+            C.cast(self._during, C.c_void_p).value if call else None)
+
     def __getitem__(self, name: str) -> int:
         return self._state[SLOTS.index(name)]
 

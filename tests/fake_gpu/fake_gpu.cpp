@@ -33,6 +33,7 @@ enum {
 };
 extern "C" {
 int64_t fake_state[kSlots] = {INT64_MAX, INT64_MAX};
+void (*fake_during)() = nullptr;  // called while a counting kernel runs
 void fake_reset();
 int fake_from_csr_device(int32_t V, int64_t E, const int64_t *off, const int32_t *adj);
 }
@@ -89,8 +90,9 @@ cudaError_t give(void *p) {
     return cudaSuccess;
 }
 
-// Every array of a graph that a kernel is handed.
+// Every array of a graph that a counting kernel is handed.
 void check(const DevGraphView &g, bool bitmaps) {
+    if (fake_during) fake_during();
     need(g.off, 8 * (size_t(g.V) + 1));
     need(g.lo_off, 8 * (size_t(g.V) + 1));
     need(g.adj, 4 * size_t(g.E));

@@ -104,3 +104,47 @@ def test_five_cycles_without_bitmaps(gat, on_fake):
         cfg.hub_bitmaps = flag
         for how in _counted(gat, g, cfg):
             assert on_fake["c5_bitmaps"] == flag, how
+
+
+UPLOADS = [dict(hub_min_degree=0), dict(degree_order=False), dict(hub_min_degree=20), dict()]
+
+
+def test_batches_keep_their_arrays(gat, on_fake):
+    """A prepared batch counts on the arrays it was prepared with, whatever
+    its graphs' later uploads let go of; nothing stays behind the batch."""
+    g = gat.Graph.barabasi_albert(500, 4, 1)
+    g.upload()
+    live = on_fake["live"]
+    b = gat.Batch()
+    for p, mode in ((C5, "exact"), (HOUSE, "exact"), (HOUSE, "ref")):
+        b.add(g, gat.Schedule(p, mode))
+    b.prepare(cuda_graph=False)
+    for again in UPLOADS:
+        g.upload(**again)
+        b.run()
+        assert on_fake["misuse"] == 0, again
+    del b
+    gc.collect()
+    g.upload()
+    assert on_fake["live"] == live
+    del g
+    gc.collect()
+    assert on_fake["live"] == 0
+
+
+@pytest.mark.parametrize("pattern,mode", [(C5, "exact"), (K4, "exact"), (C4, "exact"),
+                                          (HOUSE, "exact"), (HOUSE, "ref")])
+def test_counts_keep_their_arrays(gat, on_fake, pattern, mode):
+    """A graph uploaded again by another thread while a count runs."""
+    g = gat.Graph.barabasi_albert(500, 4, 1)
+    ex, s = gat.Executor(), gat.Schedule(pattern, mode)
+    try:
+        for again in UPLOADS:
+            g.upload()
+            ex.count(g, s)  # (the given-id copy's bitmaps are made on first use)
+            on_fake.during(lambda: g.upload(**again))
+            ex.count(g, s)
+            on_fake.during(None)
+            assert on_fake["misuse"] == 0, again
+    finally:
+        on_fake.during(None)
