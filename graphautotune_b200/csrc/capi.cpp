@@ -871,6 +871,7 @@ int gat_graph_from_csr_device(int32_t V, int64_t E, const int64_t *offsets,
     *out = nullptr;
     cudaStream_t st = (cudaStream_t)stream;
     auto g = std::make_unique<gat_graph>();
+    g->host.off.reserve(size_t(V) + 1);
     DevCopy &d = g->dev;
     unsigned long long *flag = nullptr;
     cudaError_t e;
@@ -885,7 +886,8 @@ int gat_graph_from_csr_device(int32_t V, int64_t E, const int64_t *offsets,
     h.V = V;
     h.E = E;
     unsigned long long bad = ~0ull;
-    // the host's copy of the offsets is made while the device works
+    // the host's copy of the offsets is made while the device works, in room
+    // that is there before
     auto keep_offsets = [&] { h.off.assign(offsets, offsets + size_t(V) + 1); };
     if ((e = cudaMemcpyAsync(d.off, offsets, sizeof(int64_t) * (size_t(V) + 1),
                              cudaMemcpyHostToDevice, st)) != cudaSuccess ||

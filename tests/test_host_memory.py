@@ -148,3 +148,21 @@ def test_counts_keep_their_arrays(gat, on_fake, pattern, mode):
             assert on_fake["misuse"] == 0, again
     finally:
         on_fake.during(None)
+
+
+def test_host_memory_runs_out_before_the_copies(gat, on_fake):
+    """A graph from host arrays whose host copy cannot be allocated: no copy
+    from the caller's arrays is on its way when the call ends."""
+    import ctypes as C
+
+    off, adj = gat.Graph.barabasi_albert(500, 4, 1).csr()
+    call = on_fake.lib.fake_from_csr_device
+    call.argtypes = [C.c_int32, C.c_int64, C.c_void_p, C.c_void_p]
+    args = (500, len(adj), off.ctypes.data, adj.ctypes.data)
+    on_fake["throw"] = off.nbytes
+    live, on_fake["pending"] = on_fake["live"], 0
+    try:
+        assert call(*args) == -1
+    finally:
+        on_fake["throw"] = fake_gpu.NEVER
+    assert on_fake["pending"] == 0 and on_fake["live"] == live
