@@ -45,6 +45,7 @@ struct Block {
     unsigned long long id;
 };
 std::map<const char *, Block> g_blocks;
+std::multimap<size_t, char *> g_dead;  // addresses a reset has left to use again
 unsigned long long g_next_id = 1;
 int64_t g_context = 1;  // a pool, stream or event of another one is dead
 
@@ -72,7 +73,9 @@ void need(const void *p, size_t bytes) {
 cudaError_t take(void **p, size_t bytes) {
     *p = nullptr;
     if ((int64_t)bytes >= fake_state[kRefuse]) return cudaErrorMemoryAllocation;
-    char *q = static_cast<char *>(std::malloc(bytes + 64));
+    auto again = g_dead.find(bytes);
+    char *q = again != g_dead.end() ? again->second : static_cast<char *>(std::malloc(bytes + 64));
+    if (again != g_dead.end()) g_dead.erase(again);
     std::memset(q, 0x5A, bytes + 64);
     g_blocks[q] = {bytes, g_next_id++};
     fake_state[kLive]++;
@@ -143,7 +146,9 @@ extern "C" {
 
 // cudaDeviceReset: every block, pool, stream and event of the context is gone.
 void fake_reset() {
-    while (!g_blocks.empty()) give(const_cast<char *>(g_blocks.begin()->first));
+    for (auto &b : g_blocks) g_dead.insert({b.second.bytes, const_cast<char *>(b.first)});
+    g_blocks.clear();
+    fake_state[kLive] = 0;
     g_context++;
 }
 

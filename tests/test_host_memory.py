@@ -112,6 +112,9 @@ UPLOADS = [dict(hub_min_degree=0), dict(degree_order=False), dict(hub_min_degree
 def test_batches_keep_their_arrays(gat, on_fake):
     """A prepared batch counts on the arrays it was prepared with, whatever
     its graphs' later uploads let go of; nothing stays behind the batch."""
+    gat.Graph.barabasi_albert(500, 4, 1).upload()
+    gc.collect()
+    none = on_fake["live"]  # (what the pool itself holds)
     g = gat.Graph.barabasi_albert(500, 4, 1)
     g.upload()
     live = on_fake["live"]
@@ -129,7 +132,7 @@ def test_batches_keep_their_arrays(gat, on_fake):
     assert on_fake["live"] == live
     del g
     gc.collect()
-    assert on_fake["live"] == 0
+    assert on_fake["live"] == none
 
 
 @pytest.mark.parametrize("pattern,mode", [(C5, "exact"), (K4, "exact"), (C4, "exact"),
@@ -166,3 +169,24 @@ def test_host_memory_runs_out_before_the_copies(gat, on_fake):
     finally:
         on_fake["throw"] = fake_gpu.NEVER
     assert on_fake["pending"] == 0 and on_fake["live"] == live
+
+
+def test_uploads_after_a_device_reset(gat, on_fake):
+    """cudaDeviceReset takes the library's pool with it, with handles alive or
+    not; the addresses are given out again."""
+    s = gat.Schedule(HOUSE, "exact")
+    old = [(gat.Executor(), gat.Graph.barabasi_albert(500, 4, 1)) for _ in range(2)]
+    old[0][0].count(old[0][1], s)
+    del old[0]
+    for _ in range(2):
+        on_fake.lib.fake_reset()
+        ex, g = gat.Executor(), gat.Graph.barabasi_albert(500, 4, 1)
+        ex.count(g, s)
+        g.upload(hub_min_degree=0)
+        ex.count(g, s)
+        assert on_fake["misuse"] == 0
+        del ex, g
+        gc.collect()
+    del old
+    gc.collect()
+    assert on_fake["misuse"] == 0
