@@ -45,6 +45,8 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <limits>
+#include <type_traits>
 
 #include "engine.hpp"
 
@@ -345,7 +347,7 @@ struct RootSmem {
     int32_t pref[BLOCK + 2];  // exclusive prefix of the lengths of its kind,
                               // each kind followed by its total
     int32_t warp_len[2][BLOCK / 32], warp_num[2][BLOCK / 32];
-    int next[2];               // next entry to take (of this group and the next)
+    unsigned next[2];          // next entry to take (of this group and the next)
     typename Reduce::TempStorage reduce;
     int64_t root;
     long long total;
@@ -478,12 +480,17 @@ __device__ __forceinline__ void each_entry(RootSmem<BLOCK> &S, const int32_t *__
     if (nlong == 0) return;
     // long segments, a piece at a time
     const int32_t piece = max(512, total / (kWarps * kPieces));
+    // every warp takes one piece past the end
+    static_assert(INT32_MAX + uint64_t(kWarps) * (INT32_MAX / (kWarps * kPieces)) <=
+                      std::numeric_limits<std::remove_reference_t<decltype(S.next[0])>>::max(),
+                  "the counter does not wrap");
     for (;;) {
-        int32_t j = 0;
-        if (lane == 0) j = atomicAdd(&S.next[b], piece);
-        j = __shfl_sync(0xffffffffu, j, 0);
-        if (j >= total) break;
-        const int32_t je = min(total, j + piece);
+        unsigned taken = 0;
+        if (lane == 0) taken = atomicAdd(&S.next[b], (unsigned)piece);
+        taken = __shfl_sync(0xffffffffu, taken, 0);
+        if (taken >= (unsigned)total) break;
+        int32_t j = (int32_t)taken;
+        const int32_t je = total - j < piece ? total : j + piece;
         // the segment holding entry j: 32-ary search of the prefixes
         const bool in0 = lane * 32 < nlong && S.pref[lane * 32] <= j;
         int s = (__popc(__ballot_sync(0xffffffffu, in0)) - 1) * 32;
