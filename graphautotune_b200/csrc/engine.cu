@@ -1135,8 +1135,10 @@ __global__ void __launch_bounds__(256, 4)
     const bool pairs = !ALL_ENTRIES && P.basic == 2 && P.lane_last;
     const int64_t tiles = (int64_t)gridDim.x * tiles_per_block;
     int64_t left = a.num_tasks - a.task_begin;
-    // (a grab of a split queue is one part of one unit)
-    const int parts = unit_parts(left, tiles, P.basic);
+    // (a grab of a split queue is one part of one unit; an instrumented launch
+    // splits none: every part forms the unit's first sets again, and the bytes
+    // are the plan's, not the launch shape's)
+    const int parts = STATS ? 1 : unit_parts(left, tiles, P.basic);
     for (;;) {
         unsigned long long start = 0;
         if (parts > 1) {
