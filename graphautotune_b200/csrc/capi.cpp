@@ -163,7 +163,6 @@ struct gat_executor {
     int sms = 0;
     int32_t *scratch = nullptr;
     size_t scratch_bytes = 0;
-    bool scratch_clean = false;  // all-zero (the 4-cycle kernel's invariant)
     int c4_light_occ[2] = {}, c4_root_occ[2][2] = {};  // CTAs per SM, 0: not asked yet
     DevCounters *ctr = nullptr;
     DevCounters *host_ctr = nullptr;  // pinned
@@ -1070,7 +1069,6 @@ int run_c4(gat_executor *e, const DevGraphView &view, const DevCopy &dc, int64_t
             return fail(GAT_ERR_MEMORY, std::string("4-cycle scratch: ") + cudaGetErrorString(ce));
         e->scratch_bytes = need;
     }
-    e->scratch_clean = false;
     unsigned char *base = reinterpret_cast<unsigned char *>(e->scratch);
     C4Launch L;
     L.g = view;
@@ -1146,7 +1144,6 @@ int run_clique(gat_executor *e, const DevGraphView &view, int64_t vb, int64_t ve
             return fail(GAT_ERR_MEMORY, std::string("clique scratch: ") + cudaGetErrorString(ce));
         e->scratch_bytes = need;
     }
-    e->scratch_clean = false;
     unsigned char *base = reinterpret_cast<unsigned char *>(e->scratch);
     CliqueLaunch L;
     L.g = view;
@@ -1376,7 +1373,6 @@ int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *strea
     int occ = blocks_per_sm(shape.tile, shape.block, balg);
     if (occ <= 0) return fail(GAT_ERR_CUDA, "kernel does not fit on the device");
     shape.grid = e->cfg.num_blocks > 0 ? e->cfg.num_blocks : e->sms * occ;
-    e->scratch_clean = false;
     const int64_t stride = tile_scratch_ints(plan, view.max_degree);
     const int64_t tiles_per_block = shape.block / shape.tile;
     const int64_t budget = e->cfg.memory_budget > 0 ? e->cfg.memory_budget : (int64_t(4) << 30);

@@ -571,7 +571,7 @@ constexpr int64_t kSmallEntries = 1 << 19;
 constexpr int64_t kFewHeavy = 64;
 
 // A CTA per root: heavy roots [heavy_begin, heavy_end) first, then the
-// deferred ones.  WIDE: 32-bit window counters (a count may reach 2^16).
+// deferred ones.
 template <int BLOCK, bool STATS>
 __global__ void __launch_bounds__(BLOCK, RootShape<BLOCK>::kCtas)
     c4_root_kernel(const RootArgs a) {

@@ -793,8 +793,10 @@ __device__ __forceinline__ long long lane_slot(const State &st, const GatPlan &P
 // has to be stored.  Each set and each IEP value is formed exactly as
 // level_sets and iep_value form it (same bounds, exclusions and choice of
 // lists).  `i` is the candidate's position in its list.  Up to kFewSets sets
-// and slots (all plans of five vertices and fewer but a few) stay in
-// registers; arrays indexed at run time live in local memory.
+// and slots (all plans of five vertices and fewer but a few) are kept as
+// scalars; arrays indexed at run time live in local memory.  (The kernels are
+// held to 64 registers for four CTAs an SM and spill 56 to 196 bytes of their
+// state; with this function out of line they spilled 320 to 860.)
 constexpr int kFewSets = 3;
 
 template <class T>
@@ -878,16 +880,15 @@ __device__ __forceinline__ unsigned heavy_lanes(const Tile<G> &t, int32_t cost) 
 // of the tile takes candidates i, i+G, ... of the level's loop list
 // src[0, n) (lane_candidate).  No shared-memory writes, no syncs, and no idle
 // lanes when the lists are shorter than the tile.  Returns the sum of the
-// candidates' IEP values on every lane.  Of `parts` slices of the list, slice
-// `part` alone (whole groups of G candidates).
+// candidates' IEP values on every lane.
 template <int G, bool STATS>
 __device__ unsigned long long lane_last_level(const Tile<G> &t, const TileSmem &S,
                                               const GatPlan &P, const SearchArgs &a, int k,
                                               unsigned long long &bytes, const int32_t *src,
-                                              int n, int part = 0, int parts = 1) {
+                                              int n) {
     const TileState st{S};
     unsigned long long sum = 0, by = 0;
-    for (int i = part * G + t.lane; i < n; i += parts * G) {
+    for (int i = t.lane; i < n; i += G) {
         const int32_t cand = src[i];
         const bool hit = collides(st, P, k, cand);
         // Exact plans skip a colliding candidate; reference plans keep it
@@ -988,14 +989,14 @@ __device__ __forceinline__ bool lane_worth(const TileSmem &S, const GatPlan &P, 
     return cnt >= fmax;
 }
 
-// (`part` of `parts`: only every parts-th level-2 candidate of the units, or
-// group of G of them where the lanes take them.)
 // Runs the level-1 units [start, end) of one job: each unit (v0, v1) is the
 // start of a depth-first walk over levels 2 .. basic-1.  Lane 0 of the tile
 // accumulates the units' IEP values in `acc`.
 // ALL_ENTRIES: units are numbered by CSR entry even when the plan bounds
 // v1 < v0, and the units that break the bound are skipped here (no
 // lower-neighbour offset table needed); used by the allocation-free path.
+// `part` of `parts`: only every parts-th level-2 candidate of the units (plans
+// of four levels and more).
 template <int G, bool STATS, bool ALL_ENTRIES>
 __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const GatPlan &P,
                                           const SearchArgs &a, int64_t start, int64_t end,
@@ -1034,8 +1035,7 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
         setup_level(t, S, P, 2);
         if (basic == 3 && P.lane_last && lane_worth<G>(S, P, 2, S.cnt[2])) {
             const unsigned long long r =
-                lane_last_level<G, STATS>(t, S, P, a, 2, bytes, S.src[2], S.cnt[2], part,
-                                          parts);
+                lane_last_level<G, STATS>(t, S, P, a, 2, bytes, S.src[2], S.cnt[2]);
             if (t.lane == 0) acc += r;
             continue;
         }
