@@ -1040,7 +1040,7 @@ namespace {
 int run_c4(gat_executor *e, const DevGraphView &view, const DevCopy &dc, int64_t vb,
            int64_t ve, LaunchShape shape, cudaStream_t strm, bool balg, uint64_t *count,
            gat_stats *stats, std::chrono::steady_clock::time_point t0) {
-    const int root_threads = c4_root_threads(view.E, dc.heavy_rows);
+    const int root_threads = c4_root_threads(view.V, view.E, dc.heavy_rows);
     // (asked once per executor: the device does not change under it)
     int &locc = e->c4_light_occ[balg], &rocc = e->c4_root_occ[balg][root_threads == 1024];
     if (locc <= 0) locc = c4_light_blocks_per_sm(balg);

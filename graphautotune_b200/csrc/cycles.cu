@@ -201,9 +201,14 @@ struct LightArgs {
     int32_t mark[kMarks];  // window ends (V: none), and where every row passes
     int32_t *marks;        // them: kMarks x V positions
     int32_t most;          // wedges of a root that its warp counts itself
+    int32_t chunk;         // roots a grab
 };
 
-// A warp per root of [v_begin, v_end), roots handed out one at a time.
+// A warp per root of [v_begin, v_end), handed out one at a time, or, where the
+// warps get many each, up to kMostRoots: on trees the grabs were a fifth of the
+// count (Barabasi-Albert 200,000 x 1).
+constexpr int64_t kRootShare = 16;  // grabs a warp, about
+constexpr int64_t kMostRoots = 8;
 constexpr size_t kLightSmem = size_t(kLightBlock / 32) * kWarpSlots * 8;
 
 template <bool STATS>
@@ -228,89 +233,92 @@ __global__ void __launch_bounds__(kLightBlock) c4_light_kernel(const LightArgs a
     unsigned long long part = 0, bytes = 0;
     for (;;) {
         unsigned long long r = 0;
-        if (lane == 0) r = atomicAdd(&a.aux->light_cursor, 1ull);
+        if (lane == 0) r = atomicAdd(&a.aux->light_cursor, (unsigned long long)a.chunk);
         r = __shfl_sync(0xffffffffu, r, 0);
-        const int64_t v0 = a.v_begin + (int64_t)r;
-        if (v0 >= a.v_end) break;
-        const int64_t o0 = a.off[v0];
-        const int32_t d0 = (int32_t)(a.off[v0 + 1] - o0);
-        const int32_t lo0 = (int32_t)(a.lo_off[v0 + 1] - a.lo_off[v0]);
-        if (d0 - lo0 < 2) continue;  // a cycle needs two neighbours above v0
-        // This lane's upper neighbour of a group of 32: where its list rises
-        // above v0, and how many entries that leaves.
-        auto segment = [&](int i, int64_t &at) -> int32_t {
-            if (i >= d0) return 0;
-            const int32_t v1 = a.adj[o0 + i];
-            const int64_t o1 = a.off[v1];
-            const int32_t d1 = (int32_t)(a.off[v1 + 1] - o1);
-            const int32_t s1 = above(a.adj + o1, a.lo_off, v1, (int32_t)v0);
-            at = o1 + s1;
-            return d1 - s1;
-        };
-        // wedges of this root: sum over upper neighbours of |N(v1) above v0|
-        int32_t wl = 0, len = 0;
-        int64_t at = 0;
-        for (int i0 = lo0; i0 < d0; i0 += 32) {
-            len = segment(i0 + lane, at);
-            wl += len;
-        }
-        const int32_t W = __reduce_add_sync(0xffffffffu, wl);
-        if (W > a.most) {
-            if (lane == 0) {
-                const unsigned long long slot = atomicAdd(&a.aux->deferred_count, 1ull);
-                a.deferred[slot] = (int32_t)v0;
+        const int64_t first = a.v_begin + (int64_t)r;
+        if (first >= a.v_end) break;
+        const int64_t last = min(first + a.chunk, a.v_end);
+        for (int64_t v0 = first; v0 < last; v0++) {
+            const int64_t o0 = a.off[v0];
+            const int32_t d0 = (int32_t)(a.off[v0 + 1] - o0);
+            const int32_t lo0 = (int32_t)(a.lo_off[v0 + 1] - a.lo_off[v0]);
+            if (d0 - lo0 < 2) continue;  // a cycle needs two neighbours above v0
+            // This lane's upper neighbour of a group of 32: where its list rises
+            // above v0, and how many entries that leaves.
+            auto segment = [&](int i, int64_t &at) -> int32_t {
+                if (i >= d0) return 0;
+                const int32_t v1 = a.adj[o0 + i];
+                const int64_t o1 = a.off[v1];
+                const int32_t d1 = (int32_t)(a.off[v1 + 1] - o1);
+                const int32_t s1 = above(a.adj + o1, a.lo_off, v1, (int32_t)v0);
+                at = o1 + s1;
+                return d1 - s1;
+            };
+            // wedges of this root: sum over upper neighbours of |N(v1) above v0|
+            int32_t wl = 0, len = 0;
+            int64_t at = 0;
+            for (int i0 = lo0; i0 < d0; i0 += 32) {
+                len = segment(i0 + lane, at);
+                wl += len;
             }
-            continue;
-        }
-        if (W < 2) continue;
-        // A table of four slots a wedge and more where the warp's room has
-        // them: it is read out whole.
-        const int bits = min(kWarpBits, max(5, 32 - __clz(4 * W - 1)));
-        for (int i0 = lo0; i0 < d0; i0 += 32) {
-            if (d0 - lo0 > 32) len = segment(i0 + lane, at);  // else known from above
-            constexpr int kAhead = 4;
-            // The group's entries laid end to end, the lanes on consecutive
-            // ones: entry j belongs to the last lane whose exclusive prefix is
-            // at most j.  (A lane walking its own list takes as long as the
-            // longest: 34 us for 1,500 roots with a hub's list among theirs,
-            // 24 so; on a uniform G(30,000, 20) 146 us a count against 126.)
-            int32_t pre = len;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int32_t y = __shfl_up_sync(0xffffffffu, pre, o);
-                if (lane >= o) pre += y;
-            }
-            const int32_t total = __shfl_sync(0xffffffffu, pre, 31);
-            pre -= len;
-            for (int32_t j0 = 0; j0 < total; j0 += 32 * kAhead) {
-                int32_t xs[kAhead];
-#pragma unroll
-                for (int u = 0; u < kAhead; u++) {
-                    const int32_t j = j0 + 32 * u + lane;
-                    int own = 0;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1)
-                        if (__shfl_sync(0xffffffffu, pre, own + o) <= j) own += o;
-                    const int64_t from = __shfl_sync(0xffffffffu, at, own);
-                    const int32_t first = __shfl_sync(0xffffffffu, pre, own);
-                    xs[u] = j < total ? __ldg(a.adj + from + (j - first)) : 0;
+            const int32_t W = __reduce_add_sync(0xffffffffu, wl);
+            if (W > a.most) {
+                if (lane == 0) {
+                    const unsigned long long slot = atomicAdd(&a.aux->deferred_count, 1ull);
+                    a.deferred[slot] = (int32_t)v0;
                 }
-#pragma unroll
-                for (int u = 0; u < kAhead; u++)
-                    if (xs[u] > 0) table_add(key, cnt, bits, xs[u], &a.ctr->error);
+                continue;
             }
-            if (STATS && i0 + lane < d0) bytes += 20;
-        }
-        if (STATS) bytes += 4ull * (unsigned)wl;
-        __syncwarp();
-        for (int i = lane; i < (1 << bits); i += 32) {
-            if (key[i] != kEmpty) {
-                part += pairs_of(cnt[i]);
-                key[i] = kEmpty;
-                cnt[i] = 0;
+            if (W < 2) continue;
+            // A table of four slots a wedge and more where the warp's room has
+            // them: it is read out whole.
+            const int bits = min(kWarpBits, max(5, 32 - __clz(4 * W - 1)));
+            for (int i0 = lo0; i0 < d0; i0 += 32) {
+                if (d0 - lo0 > 32) len = segment(i0 + lane, at);  // else known from above
+                constexpr int kAhead = 4;
+                // The group's entries laid end to end, the lanes on consecutive
+                // ones: entry j belongs to the last lane whose exclusive prefix is
+                // at most j.  (A lane walking its own list takes as long as the
+                // longest: 34 us for 1,500 roots with a hub's list among theirs,
+                // 24 so; on a uniform G(30,000, 20) 146 us a count against 126.)
+                int32_t pre = len;
+    #pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int32_t y = __shfl_up_sync(0xffffffffu, pre, o);
+                    if (lane >= o) pre += y;
+                }
+                const int32_t total = __shfl_sync(0xffffffffu, pre, 31);
+                pre -= len;
+                for (int32_t j0 = 0; j0 < total; j0 += 32 * kAhead) {
+                    int32_t xs[kAhead];
+    #pragma unroll
+                    for (int u = 0; u < kAhead; u++) {
+                        const int32_t j = j0 + 32 * u + lane;
+                        int own = 0;
+    #pragma unroll
+                        for (int o = 16; o > 0; o >>= 1)
+                            if (__shfl_sync(0xffffffffu, pre, own + o) <= j) own += o;
+                        const int64_t from = __shfl_sync(0xffffffffu, at, own);
+                        const int32_t first = __shfl_sync(0xffffffffu, pre, own);
+                        xs[u] = j < total ? __ldg(a.adj + from + (j - first)) : 0;
+                    }
+    #pragma unroll
+                    for (int u = 0; u < kAhead; u++)
+                        if (xs[u] > 0) table_add(key, cnt, bits, xs[u], &a.ctr->error);
+                }
+                if (STATS && i0 + lane < d0) bytes += 20;
             }
+            if (STATS) bytes += 4ull * (unsigned)wl;
+            __syncwarp();
+            for (int i = lane; i < (1 << bits); i += 32) {
+                if (key[i] != kEmpty) {
+                    part += pairs_of(cnt[i]);
+                    key[i] = kEmpty;
+                    cnt[i] = 0;
+                }
+            }
+            __syncwarp();
         }
-        __syncwarp();
     }
     for (int o = 16; o > 0; o >>= 1) {
         part += __shfl_xor_sync(0xffffffffu, part, o);
@@ -566,9 +574,13 @@ __device__ __forceinline__ int table_bits(long long W) {
 // Graphs of fewer directed entries and at least this many heavy roots take
 // the CTAs of 1,024 threads (R-MAT 2^15: 193 us a count against 236;
 // Barabasi-Albert 20,000 x 9, 25 heavy roots and thousands of small ones, 164
-// against 142).
-constexpr int64_t kSmallEntries = 1 << 19;
-constexpr int64_t kFewHeavy = 64;
+// against 142), and so do larger ones with a dense core (R-MAT 2^17 with 15
+// entries a vertex: 629 us against 728; with 7.6: 360 against 343;
+// Barabasi-Albert 65,000 x 9, 88 heavy roots: 338 against 251; R-MAT 2^18 with
+// 11: 1,008 either way).
+constexpr int64_t kSmallEntries = 1 << 19, kMiddleEntries = 1 << 21;
+constexpr int64_t kFewHeavy = 64, kCoreHeavy = 512;
+constexpr int64_t kCoreDensity = 10;  // entries a vertex
 
 // A CTA per root: heavy roots [heavy_begin, heavy_end) first, then the
 // deferred ones.
@@ -784,8 +796,11 @@ int c4_light_blocks_per_sm(bool stats) {
     return stats ? light_occupancy<true>() : light_occupancy<false>();
 }
 
-int c4_root_threads(int64_t E, int64_t heavy_rows) {
-    return E < kSmallEntries && heavy_rows >= kFewHeavy ? 1024 : 512;
+int c4_root_threads(int32_t V, int64_t E, int64_t heavy_rows) {
+    const bool small = E < kSmallEntries && heavy_rows >= kFewHeavy;
+    const bool core =
+        E < kMiddleEntries && heavy_rows >= kCoreHeavy && E >= kCoreDensity * V;
+    return small || core ? 1024 : 512;
 }
 
 int c4_root_blocks_per_sm(int threads, bool stats) {
@@ -816,7 +831,9 @@ cudaError_t launch_c4(const C4Launch &L, cudaStream_t st) {
     const bool roots = L.v_begin < L.v_end;
     if (lb < le || (roots && marked)) {
         LightArgs la{g.off, g.adj, g.lo_off, lb, le, L.ctr, L.aux, L.deferred, g.V, {}, L.marks,
-                     warp_wedges(g.V)};
+                     warp_wedges(g.V), 1};
+        const int64_t share = (le - lb) / (int64_t(L.light_grid) * (kLightBlock / 32) * kRootShare);
+        la.chunk = (int32_t)std::min(std::max<int64_t>(share, 1), kMostRoots);
         for (int m = 0; m < kMarks; m++) la.mark[m] = mark[m];
         if ((e = L.stats ? light_attr<true>() : light_attr<false>()) != cudaSuccess) return e;
         if (L.stats)

@@ -113,7 +113,7 @@ struct C4Launch {
 int64_t c4_mark_ints(int32_t V);
 int c4_light_blocks_per_sm(bool stats);
 // threads of the root kernel's CTAs on this graph
-int c4_root_threads(int64_t E, int64_t heavy_rows);
+int c4_root_threads(int32_t V, int64_t E, int64_t heavy_rows);
 int c4_root_blocks_per_sm(int threads, bool stats);
 cudaError_t launch_c4(const C4Launch &launch, cudaStream_t st);
 

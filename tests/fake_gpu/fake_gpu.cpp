@@ -357,7 +357,7 @@ cudaError_t launch_clique(const CliqueLaunch &l, cudaStream_t) {
 
 int64_t c4_mark_ints(int32_t V) { return 2 * int64_t(V); }
 int c4_light_blocks_per_sm(bool) { return 2; }
-int c4_root_threads(int64_t, int64_t) { return 512; }
+int c4_root_threads(int32_t, int64_t, int64_t) { return 512; }
 int c4_root_blocks_per_sm(int, bool) { return 2; }
 cudaError_t launch_c4(const C4Launch &l, cudaStream_t) {
     check(l.g, false);
