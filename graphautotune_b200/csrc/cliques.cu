@@ -902,14 +902,24 @@ __global__ void __launch_bounds__(kCtaThreads, 2) clique_cta_kernel(const Clique
     flush_totals(a, c, bytes, STATS, lane);
 }
 
+constexpr int32_t kShortLists = 8;  // longest lower list
+constexpr int kShortChunk = 8;
+
 template <int K, bool STATS>
-cudaError_t launch_k(const CliqueArgs &a, int warp_grid, int cta_grid, cudaStream_t st) {
+cudaError_t launch_k(const CliqueArgs &a, int32_t max_lower, int warp_grid, int cta_grid,
+                     cudaStream_t st) {
     cudaError_t e;
     // ids per grab: up to 32 are looked at in one go, but no more than 1/32 of
     // a warp's share: neighbouring ids have lists of like length, and the
-    // long ones must spread over the grid
-    const int64_t share = (a.v_end - a.v_begin) / (int64_t(warp_grid) * (kWarpThreads / 32) * 32);
-    const int chunk = (int)std::min<int64_t>(std::max<int64_t>(share, 1), kRootChunk);
+    // long ones must spread over the grid.  Where all lists are short there is
+    // little to spread, and a grab costs more than the ids in it: a share, up
+    // to kShortChunk (Barabasi-Albert 200,000 x 1: 0.150 ms a count with a grab
+    // an id, 0.04 so; 2^20 x 4, 5-cliques: 0.76 at 3 ids, 0.83 at 32)
+    const bool few = max_lower <= kShortLists;
+    const int64_t share =
+        (a.v_end - a.v_begin) / (int64_t(warp_grid) * (kWarpThreads / 32) * (few ? 1 : 32));
+    const int chunk =
+        (int)std::min<int64_t>(std::max<int64_t>(share, 1), few ? kShortChunk : kRootChunk);
     clique_warp_kernel<K, STATS><<<warp_grid, kWarpThreads, 0, st>>>(a, chunk);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const size_t cs = sizeof(CtaSmem<K>);
@@ -982,14 +992,14 @@ cudaError_t launch_clique(const CliqueLaunch &L, cudaStream_t st) {
         a.list_at[b] = a.list_at[b - 1] + list_room(b - 1, g.lo_total);
     if (L.v_end <= L.v_begin) return cudaSuccess;
     switch (L.k * 2 + (L.stats ? 1 : 0)) {
-        case 8: return launch_k<4, false>(a, L.warp_grid, L.cta_grid, st);
-        case 9: return launch_k<4, true>(a, L.warp_grid, L.cta_grid, st);
-        case 10: return launch_k<5, false>(a, L.warp_grid, L.cta_grid, st);
-        case 11: return launch_k<5, true>(a, L.warp_grid, L.cta_grid, st);
-        case 12: return launch_k<6, false>(a, L.warp_grid, L.cta_grid, st);
-        case 13: return launch_k<6, true>(a, L.warp_grid, L.cta_grid, st);
-        case 14: return launch_k<7, false>(a, L.warp_grid, L.cta_grid, st);
-        case 15: return launch_k<7, true>(a, L.warp_grid, L.cta_grid, st);
+        case 8: return launch_k<4, false>(a, g.max_lower, L.warp_grid, L.cta_grid, st);
+        case 9: return launch_k<4, true>(a, g.max_lower, L.warp_grid, L.cta_grid, st);
+        case 10: return launch_k<5, false>(a, g.max_lower, L.warp_grid, L.cta_grid, st);
+        case 11: return launch_k<5, true>(a, g.max_lower, L.warp_grid, L.cta_grid, st);
+        case 12: return launch_k<6, false>(a, g.max_lower, L.warp_grid, L.cta_grid, st);
+        case 13: return launch_k<6, true>(a, g.max_lower, L.warp_grid, L.cta_grid, st);
+        case 14: return launch_k<7, false>(a, g.max_lower, L.warp_grid, L.cta_grid, st);
+        case 15: return launch_k<7, true>(a, g.max_lower, L.warp_grid, L.cta_grid, st);
         default: return cudaErrorInvalidValue;
     }
 }
