@@ -100,6 +100,7 @@ struct DevCopy {
     uint32_t *bitmaps = nullptr;
     int32_t nhubs = 0;
     int64_t bitmap_words = 0;
+    bool deep_rows = false;  // DevGraphView::deep_rows
     // Holders of (off, adj, lo_off) and of (hub_slot, hubs, bitmaps).
     std::shared_ptr<DevArrays> rows = std::make_shared<DevArrays>(),
                                hub_rows = std::make_shared<DevArrays>();
@@ -710,9 +711,16 @@ int derive_ordered_copy(const HostGraph &h, const DevCopy &src, DevCopy &d, cuda
 // of kRowMinDegree, graphs whose hubs already exceed the limit no further
 // one.  Shorter lists than that are a few loads long either way.  House on
 // R-MAT 2^14: 18.1 ms with hub rows alone, 11.7 with these; 6-cycle with
-// chord on R-MAT 2^10 6.0 and 2.1 ms.
+// chord on R-MAT 2^10 6.0 and 2.1 ms.  Where no degree
+// reaches kShortRows and the rows do not hold a quarter of the entries, or not
+// all that qualify have one, they are left to the dedicated kernels and to
+// two-level plans: deeper plans are faster by their kernel without the rows'
+// code (reference-rule house on G(2^18, 4), 2,048 rows: 5.4 ms with them, 3.5
+// without; G(2^20, 1), a dozen rows: 2.7 and 1.9; 4-cliques of G(40,000, 24)
+// 0.097 ms with, 0.134 without).
 constexpr int64_t kSmallRowBytes = int64_t(64) << 20;
 constexpr int64_t kRowMinDegree = 8;
+constexpr int64_t kShortRows = 64;
 
 int build_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes, bool ordered,
                const HostGraph &h, cudaStream_t st) {
@@ -725,9 +733,9 @@ int build_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes, boo
     // Rows in decreasing order of degree: on the degree-ordered copy the
     // leading ids themselves, so only the counts are needed.
     std::vector<int32_t> cand;
-    int64_t nhubs = 0, nrows = 0;
+    int64_t nhubs = 0, nrows = 0, entries = 0;  // entries: of rows that are all there
     if (ordered) {
-        int64_t *dn = nullptr, n[2] = {0, 0};
+        int64_t *dn = nullptr, n[4] = {};  // rows and entries, twice
         if ((e = dev_alloc((void **)&dn, sizeof(n), st)) != cudaSuccess)
             return fail(GAT_ERR_MEMORY, std::string("hub bitmap allocation: ") + cudaGetErrorString(e));
         if ((e = leading_rows_device(d.off, V, min_degree, kRowMinDegree, dn, st)) != cudaSuccess ||
@@ -738,7 +746,9 @@ int build_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes, boo
         }
         dev_free(dn, st);
         nhubs = std::min(n[0], fit);
-        nrows = std::max(nhubs, n[0] < room ? std::min(std::max(n[0], n[1]), room) : 0);
+        if (n[0] < room) nrows = std::min(std::max(n[0], n[2]), room);
+        nrows = std::max(nhubs, nrows);
+        entries = nrows < n[2] ? 0 : n[3];
     } else {
         auto by_degree = [&](int32_t x, int32_t y) { return h.degree(x) > h.degree(y); };
         for (int32_t v = 0; v < V; v++)
@@ -752,6 +762,8 @@ int build_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes, boo
             nrows = std::min((int64_t)cand.size(), room);
         }
         nrows = std::max(nhubs, nrows);
+        if (nrows == (int64_t)cand.size())
+            for (int32_t v : cand) entries += h.degree(v);
         cand.resize(size_t(nrows));
     }
     if (nrows == 0) return GAT_OK;
@@ -770,6 +782,7 @@ int build_hubs(DevCopy &d, int32_t V, int64_t min_degree, int64_t max_bytes, boo
         return cuda_fail(e, "hub bitmaps");
     d.nhubs = (int32_t)nhubs;
     d.bitmap_words = words;
+    d.deep_rows = d.max_degree >= kShortRows || entries >= h.E / 4;
     return GAT_OK;
 }
 
@@ -1288,6 +1301,7 @@ int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *strea
     view.hub_slot = dc->hub_slot;
     view.bitmaps = dc->bitmaps;
     view.bitmap_words = dc->bitmap_words;
+    view.deep_rows = dc->deep_rows;
 
     LaunchShape shape;
     shape.tile = e->cfg.set_intersection_type == 1 ? 1 : e->cfg.threads_per_warp;
@@ -1370,7 +1384,9 @@ int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *strea
     // (instrumented counts, root ranges and shards follow the plan)
     if (!balg && !ranged && s->five_cycle && e->cfg.special_kernels == 1 && c5_fits(view))
         return run_c5(e, c5_view(e->cfg, view), strm, count, stats, t0);
-    int occ = blocks_per_sm(shape.tile, shape.block, balg);
+    *e->h_plan = plan;
+    if (e->cfg.special_kernels == 0) e->h_plan->lane_last = 0;
+    int occ = blocks_per_sm(*e->h_plan, view, shape, balg);
     if (occ <= 0) return fail(GAT_ERR_CUDA, "kernel does not fit on the device");
     shape.grid = e->cfg.num_blocks > 0 ? e->cfg.num_blocks : e->sms * occ;
     const int64_t stride = tile_scratch_ints(plan, view.max_degree);
@@ -1393,13 +1409,11 @@ int count_impl(gat_executor *e, gat_graph *g, const gat_schedule *s, void *strea
             return fail(GAT_ERR_MEMORY, std::string("scratch allocation: ") + cudaGetErrorString(ce));
         e->scratch_bytes = need;
     }
-    *e->h_plan = plan;
-    if (e->cfg.special_kernels == 0) e->h_plan->lane_last = 0;
     if ((ce = cudaMemcpyAsync(e->d_plan, e->h_plan, sizeof(GatPlan), cudaMemcpyHostToDevice,
                               strm)) != cudaSuccess)
         return cuda_fail(ce, "plan upload");
     cudaEventRecord(e->ev0, strm);
-    ce = launch_search(e->d_plan, plan, view, shape, e->scratch, stride, e->ctr, balg, strm);
+    ce = launch_search(e->d_plan, *e->h_plan, view, shape, e->scratch, stride, e->ctr, balg, strm);
     if (ce != cudaSuccess) return cuda_fail(ce, "search launch");
     cudaEventRecord(e->ev1, strm);
     if ((ce = cudaMemcpyAsync(e->host_ctr, e->ctr, sizeof(DevCounters), cudaMemcpyDeviceToHost,
@@ -1682,6 +1696,7 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
         v.hub_slot = dc.hub_slot;
         v.bitmaps = dc.bitmaps;
         v.bitmap_words = dc.bitmap_words;
+        v.deep_rows = dc.deep_rows;
         b->divisors[j] = s->plan.plan.divisor;
         b->modes[j] = s->mode;
         if (s->five_cycle && b->jobs[j].num_shards == 0 && b->cfg.special_kernels == 1 &&
@@ -1718,6 +1733,7 @@ int gat_batch_prepare(gat_batch *b, const gat_config *c, int use_cuda_graph) {
     for (q = 0; q < b->queued; q++) {
         vstart[q] = b->vtotal;
         b->vtotal += batch_job_grabs(host_jobs.data() + q * jb, plans[order[q]],
+                                     b->jobs[order[q]].g->host.E,
                                      int64_t(b->grid) * (b->block / b->tile), b->tile, b->chunk);
     }
     b->scratch_bytes = size_t(std::max<int64_t>(per_block * b->grid, 4));

@@ -51,7 +51,8 @@ struct TileSmem {
     int32_t pos[GAT_MAX_VERTICES];
     int32_t sl[GAT_MAX_PREFIX];
     int32_t owner[GAT_MAX_PREFIX];  // ALIAS sets: the vertex whose list it is
-    int32_t pad[2];
+    int32_t first2, step2;  // level-2 candidates of the unit in hand: from
+                            // first2 on, every step2-th
     const int32_t *src[GAT_MAX_VERTICES];
     const int32_t *sp[GAT_MAX_PREFIX];
 };
@@ -70,6 +71,8 @@ struct SearchArgs {
     int64_t scratch_stride;
     int32_t chunk;
     int32_t linear_below;
+    int32_t max_lower;
+    int32_t pad;
     const int32_t *hub_slot;   // null: no bitmaps
     const uint32_t *bitmaps;
     int64_t bitmap_words;
@@ -390,10 +393,17 @@ __device__ __forceinline__ int32_t cut_neighbours(const Tile<G> &t, const Search
     return tile_bound<G, false>(t, nb, dv, T);
 }
 
+// v's bitmap row, or -1.
+template <bool ROWS>
+__device__ __forceinline__ int row_of(const SearchArgs &a, int32_t v) {
+    return ROWS && a.hub_slot != nullptr ? a.hub_slot[v] : -1;
+}
+
 // Builds every prefix set that ends at level k for candidate v.  `cand_idx`
 // is v's position in the list it was drawn from (the loop set of level k),
 // or -1: that list cut at v is exactly its first cand_idx elements.
-template <int G, bool STATS>
+// ROWS: vertices may have bitmap rows.
+template <int G, bool STATS, bool ROWS>
 __device__ void level_sets(const Tile<G> &t, TileSmem &S, const GatPlan &P,
                            const SearchArgs &a, int k, int32_t v, bool collided,
                            int32_t *scratch, unsigned long long &bytes, int cand_idx = -1) {
@@ -401,7 +411,7 @@ __device__ void level_sets(const Tile<G> &t, TileSmem &S, const GatPlan &P,
     const int32_t *nb = a.adj + o;
     const int32_t dv = (int32_t)(a.off[v + 1] - o);
     const int pe = P.l_pbegin[k + 1];
-    const int hub_v = (a.hub_slot != nullptr) ? a.hub_slot[v] : -1;
+    const int hub_v = row_of<ROWS>(a, v);
     for (int p = P.l_pbegin[k]; p < pe; p++) {
         const int kind = P.p_kind[p];
         const int32_t *ptr = S.sp[p];
@@ -433,8 +443,7 @@ __device__ void level_sets(const Tile<G> &t, TileSmem &S, const GatPlan &P,
                 // owner's full row is a member of F.  Probing F into v's row
                 // when F is no longer than N(v) needs no cut of N(v) at all.
                 const int owner_f = S.owner[f];
-                const int hub_f =
-                    (a.hub_slot != nullptr && owner_f >= 0) ? a.hub_slot[owner_f] : -1;
+                const int hub_f = owner_f >= 0 ? row_of<ROWS>(a, owner_f) : -1;
                 const uint32_t *row = nullptr;
                 const int32_t *probe = nullptr;
                 int np = 0;
@@ -501,7 +510,7 @@ __device__ __forceinline__ void setup_level(const Tile<G> &t, TileSmem &S,
     if (t.lane == 0) {
         S.src[k] = ptr;
         S.cnt[k] = cnt;
-        S.pos[k] = 0;
+        S.pos[k] = k == 2 ? S.first2 : 0;
     }
     t.sync();
 }
@@ -681,7 +690,7 @@ __device__ __forceinline__ int and_rows(const uint32_t *x, const uint32_t *y, in
 // bounds and exclusions of level_sets.  Both lists have rows: their words
 // below the bound are ANDed when that is less work than the probes (about 3.5
 // instructions a word against 6 an element).
-template <bool STATS, class State>
+template <bool STATS, bool ROWS, class State>
 __device__ __forceinline__ int lane_set(const State &st, const GatPlan &P, const SearchArgs &a,
                                         int k, int p, int32_t cand, int i, const int32_t *nb,
                                         int32_t dv, int hub_v, unsigned long long &by) {
@@ -700,7 +709,7 @@ __device__ __forceinline__ int lane_set(const State &st, const GatPlan &P, const
             fl = lower_serial(fp, fl, T);
     }
     const int owner_f = st.owner(f);
-    const int hub_f = (a.hub_slot != nullptr && owner_f >= 0) ? a.hub_slot[owner_f] : -1;
+    const int hub_f = owner_f >= 0 ? row_of<ROWS>(a, owner_f) : -1;
     const uint32_t *row = nullptr;
     const int32_t *probe = nullptr;
     int np = 0;
@@ -792,11 +801,11 @@ __device__ __forceinline__ long long lane_slot(const State &st, const GatPlan &P
 // whose father F belongs to an earlier level or N(cand) itself, so nothing
 // has to be stored.  Each set and each IEP value is formed exactly as
 // level_sets and iep_value form it (same bounds, exclusions and choice of
-// lists).  `i` is the candidate's position in its list.  Up to kFewSets sets
-// and slots (all plans of five vertices and fewer but a few) are kept as
-// scalars; arrays indexed at run time live in local memory.  (The kernels are
-// held to 64 registers for four CTAs an SM and spill 56 to 196 bytes of their
-// state; with this function out of line they spilled 320 to 860.)
+// lists).  `i` is the candidate's position in its list.  FEW: up to kFewSets
+// sets and slots are kept as scalars; more, and all without FEW, in local
+// memory.  Only two-level plans have kernels that are short enough for both
+// (three-level gem on G(2^18, 4) 2.24 ms with, 2.10 without; two-level diamond
+// by the reference's rules on Barabasi-Albert 65,536 x 8 0.098 and 0.106).
 constexpr int kFewSets = 3;
 
 template <class T>
@@ -804,7 +813,7 @@ __device__ __forceinline__ T pick(int i, T x0, T x1, T x2) {
     return i == 0 ? x0 : i == 1 ? x1 : x2;
 }
 
-template <bool STATS, class State>
+template <bool STATS, bool ROWS, bool FEW, class State>
 __device__ __forceinline__ unsigned long long lane_candidate(const State &st, const GatPlan &P,
                                                              const SearchArgs &a, int k,
                                                              int32_t cand, int i, bool hit,
@@ -813,7 +822,7 @@ __device__ __forceinline__ unsigned long long lane_candidate(const State &st, co
     const int64_t o = a.off[cand];
     const int32_t *nb = a.adj + o;
     const int32_t dv = (int32_t)(a.off[cand + 1] - o);
-    const int hub_v = (a.hub_slot != nullptr) ? a.hub_slot[cand] : -1;
+    const int hub_v = row_of<ROWS>(a, cand);
     unsigned long long local = 0, cur = 1;
     int last = -1;
     auto term = [&](int g, unsigned long long v) {
@@ -823,10 +832,10 @@ __device__ __forceinline__ unsigned long long lane_candidate(const State &st, co
             local += cur * (unsigned long long)(long long)P.t_coef[g];
         }
     };
-    if (pe - pb <= kFewSets && P.iep_num <= kFewSets) {
+    if (FEW && pe - pb <= kFewSets && P.iep_num <= kFewSets) {
         int32_t l0 = 0, l1 = 0, l2 = 0;  // level-k sets: count, or cut length of N(cand)
         for (int p = pb; p < pe && !hit; p++) {
-            const int32_t c = lane_set<STATS>(st, P, a, k, p, cand, i, nb, dv, hub_v, by);
+            const int32_t c = lane_set<STATS, ROWS>(st, P, a, k, p, cand, i, nb, dv, hub_v, by);
             if (p == pb)
                 l0 = c;
             else if (p == pb + 1)
@@ -853,7 +862,7 @@ __device__ __forceinline__ unsigned long long lane_candidate(const State &st, co
     long long val[8];
     for (int p = pb; p < pe; p++)
         lv[p - pb] =
-            hit ? 0 : lane_set<STATS>(st, P, a, k, p, cand, i, nb, dv, hub_v, by);
+            hit ? 0 : lane_set<STATS, ROWS>(st, P, a, k, p, cand, i, nb, dv, hub_v, by);
     for (int x = 0; x < P.iep_num; x++) {
         const int at = P.iep_prefix[x] - pb;
         val[x] = lane_slot(st, P, a, k, x, cand, nb, at >= 0 && at < pe - pb ? lv[at] : 0);
@@ -881,7 +890,7 @@ __device__ __forceinline__ unsigned heavy_lanes(const Tile<G> &t, int32_t cost) 
 // src[0, n) (lane_candidate).  No shared-memory writes, no syncs, and no idle
 // lanes when the lists are shorter than the tile.  Returns the sum of the
 // candidates' IEP values on every lane.
-template <int G, bool STATS>
+template <int G, bool STATS, bool ROWS>
 __device__ unsigned long long lane_last_level(const Tile<G> &t, const TileSmem &S,
                                               const GatPlan &P, const SearchArgs &a, int k,
                                               unsigned long long &bytes, const int32_t *src,
@@ -894,7 +903,7 @@ __device__ unsigned long long lane_last_level(const Tile<G> &t, const TileSmem &
         // Exact plans skip a colliding candidate; reference plans keep it
         // with every level-k set empty.
         if (hit && !P.collide_clear) continue;
-        sum += lane_candidate<STATS>(st, P, a, k, cand, i, hit, by);
+        sum += lane_candidate<STATS, ROWS, false>(st, P, a, k, cand, i, hit, by);
     }
     if (STATS) {
         by = t.sum(by);
@@ -949,7 +958,7 @@ __device__ __forceinline__ void run_pairs(const Tile<G> &t, TileSmem &S, const G
         }
         unsigned heavy = heavy_lanes(t, cost);
         if (live && !((heavy >> t.lane) & 1u))
-            sum += lane_candidate<STATS>(st, P, a, 1, v1, i, hit, by);
+            sum += lane_candidate<STATS, true, true>(st, P, a, 1, v1, i, hit, by);
         while (heavy) {
             const int j = __ffs(heavy) - 1;
             heavy &= heavy - 1;
@@ -961,8 +970,8 @@ __device__ __forceinline__ void run_pairs(const Tile<G> &t, TileSmem &S, const G
                 S.v[1] = c1;
             }
             t.sync();
-            level_sets<G, STATS>(t, S, P, a, 0, c0, false, scratch, bytes);
-            level_sets<G, STATS>(t, S, P, a, 1, c1, false, scratch, bytes, ci);
+            level_sets<G, STATS, true>(t, S, P, a, 0, c0, false, scratch, bytes);
+            level_sets<G, STATS, true>(t, S, P, a, 1, c1, false, scratch, bytes, ci);
             const long long r = iep_value(t, S, P, a.linear_below);
             if (t.lane == 0) acc += (unsigned long long)r;
             t.sync();
@@ -995,19 +1004,12 @@ __device__ __forceinline__ bool lane_worth(const TileSmem &S, const GatPlan &P, 
 // ALL_ENTRIES: units are numbered by CSR entry even when the plan bounds
 // v1 < v0, and the units that break the bound are skipped here (no
 // lower-neighbour offset table needed); used by the allocation-free path.
-// `part` of `parts`: only every parts-th level-2 candidate of the units (plans
-// of four levels and more).
-template <int G, bool STATS, bool ALL_ENTRIES>
+template <int G, bool STATS, bool ALL_ENTRIES, bool ROWS>
 __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const GatPlan &P,
                                           const SearchArgs &a, int64_t start, int64_t end,
                                           int32_t *scratch, unsigned long long &acc,
-                                          unsigned long long &bytes, int part = 0,
-                                          int parts = 1) {
+                                          unsigned long long &bytes) {
     const int basic = P.basic;
-    if (!ALL_ENTRIES && basic == 2 && P.lane_last) {
-        run_pairs<G, STATS>(t, S, P, a, start, end, scratch, acc, bytes);
-        return;
-    }
     const int64_t *task_off = (!ALL_ENTRIES && P.level1_bounded) ? a.lo_off : a.off;
     int32_t row = tile_bound<G, true, int64_t>(t, task_off, a.V + 1, start) - 1;
     int32_t cur_v0 = -1;
@@ -1019,12 +1021,12 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
         if (v0 != cur_v0) {
             if (t.lane == 0) S.v[0] = v0;
             t.sync();
-            level_sets<G, STATS>(t, S, P, a, 0, v0, false, scratch, bytes);
+            level_sets<G, STATS, ROWS>(t, S, P, a, 0, v0, false, scratch, bytes);
             cur_v0 = v0;
         }
         if (t.lane == 0) S.v[1] = v1;
         t.sync();
-        level_sets<G, STATS>(t, S, P, a, 1, v1, false, scratch, bytes,
+        level_sets<G, STATS, ROWS>(t, S, P, a, 1, v1, false, scratch, bytes,
                              (int)(tk - task_off[v0]));
         if (basic == 2) {
             const long long r = iep_value(t, S, P, a.linear_below);
@@ -1035,13 +1037,9 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
         setup_level(t, S, P, 2);
         if (basic == 3 && P.lane_last && lane_worth<G>(S, P, 2, S.cnt[2])) {
             const unsigned long long r =
-                lane_last_level<G, STATS>(t, S, P, a, 2, bytes, S.src[2], S.cnt[2]);
+                lane_last_level<G, STATS, ROWS>(t, S, P, a, 2, bytes, S.src[2], S.cnt[2]);
             if (t.lane == 0) acc += r;
             continue;
-        }
-        if (parts > 1) {
-            if (t.lane == 0) S.pos[2] = part;
-            t.sync();
         }
         int k = 2;
         while (k >= 2) {
@@ -1059,14 +1057,14 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
                 hit |= (S.v[j] == cand);
             }
             t.sync();
-            if (t.lane == 0) S.pos[k] = at + (k == 2 ? parts : 1);
+            if (t.lane == 0) S.pos[k] = at + (k == 2 ? S.step2 : 1);
             if (hit && !P.collide_clear) {
                 t.sync();
                 continue;
             }
             if (t.lane == 0) S.v[k] = cand;
             t.sync();
-            level_sets<G, STATS>(t, S, P, a, k, cand, hit, scratch, bytes, at);
+            level_sets<G, STATS, ROWS>(t, S, P, a, k, cand, hit, scratch, bytes, at);
             if (k == basic - 1) {
                 const long long r = iep_value(t, S, P, a.linear_below);
                 if (t.lane == 0) acc += (unsigned long long)r;
@@ -1075,7 +1073,7 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
             }
             setup_level(t, S, P, k + 1);
             if (k + 1 == basic - 1 && P.lane_last && lane_worth<G>(S, P, k + 1, S.cnt[k + 1])) {
-                const unsigned long long r = lane_last_level<G, STATS>(
+                const unsigned long long r = lane_last_level<G, STATS, ROWS>(
                     t, S, P, a, k + 1, bytes, S.src[k + 1], S.cnt[k + 1]);
                 if (t.lane == 0) acc += r;
                 continue;
@@ -1085,42 +1083,78 @@ __device__ __forceinline__ void run_units(const Tile<G> &t, TileSmem &S, const G
     }
 }
 
+// Whether every unit of a deep plan is little work: no row is long, or the
+// level-2 candidates are an intersection on a sparse graph without a dense core.
+constexpr int kShortRows = 64;  // (largest degree)
+constexpr int kThinCore = 12;   // (longest lower list)
+constexpr int kSparse = 8, kVerySparse = 6;  // (entries a vertex)
+
+__host__ __device__ __forceinline__ bool light_units(const GatPlan &P, int32_t max_degree,
+                                                     int32_t max_lower, int32_t V, int64_t E) {
+    if (max_degree <= kShortRows) return true;
+    return P.basic >= 4 && P.p_kind[P.l_loop[2]] == GAT_SET_STORE && max_lower <= kThinCore &&
+           E < int64_t(kVerySparse) * V;
+}
+
 // Units of one queue grab.  A grab is at most `most` units (the configured
 // chunk), and shrinks with the units left to 1/share of a tile's part of
-// them: neighbouring units of hub rows are the heaviest, and a tile that
-// holds several of them runs on alone.  Grabbing unit by unit costs one
-// atomic and one row search each, which is cheap next to the walk under a
-// unit; counts of 12k to 2M units were all fastest at grabs of one
-// (6-cycle with chord on R-MAT 2^10 35.4 ms at 8 units a grab, 5.5 ms at 1;
-// two-level diamond on R-MAT 2^17 6.4 ms at 8 units a lane, 1.2 ms at 1).
+// them.  Neighbouring units of hub rows are the heaviest, and a tile that
+// holds several of them runs on alone: counts of 12k to 2M units of skewed
+// graphs were all fastest at grabs of one (6-cycle with chord on R-MAT 2^10
+// 35.4 ms at 8 units a grab, 5.5 ms at 1; two-level diamond on R-MAT 2^17 6.4 ms
+// at 8 units a lane, 1.2 ms at 1).  A grab costs an atomic and a search for its
+// row, about 2 us, which is more than a light unit: 1/64 a grab on G(2^18, 4)
+// took the triangle prism from 0.44 to 0.60 ms.  So light units are taken in
+// larger grabs, on sparse graphs until the very end, and so is every queue of
+// many units: a tile's last ones even out the heavy ones at its first.
 constexpr int kPairShare = 16;  // two-level plans: units of G at a time
-constexpr int kDeepShare = 64;
 
-__host__ __device__ __forceinline__ int64_t grab_units(int64_t left, int64_t tiles, bool pairs,
-                                                       int tile, int64_t most) {
-    const int64_t unit = pairs ? tile : 1;
-    const int64_t c = left / (tiles * (pairs ? kPairShare : kDeepShare)) / unit * unit;
-    return c < unit ? unit : (c > most ? most : c);
+__host__ __device__ __forceinline__ int grab_share(int64_t units, int64_t tiles, bool light,
+                                                   int32_t V, int64_t E) {
+    if (light) return E < int64_t(kSparse) * V && units >= 16 * tiles ? 2 : 8;
+    return units >= 128 * tiles ? 8 : 64;
+}
+
+__host__ __device__ __forceinline__ int32_t grab_units(int64_t left, int64_t tiles, int share,
+                                                       int unit, int32_t most) {
+    const int32_t c = (int32_t)fminf((float)left / (float)(tiles * share), (float)most);
+    return c <= unit ? unit : c / unit * unit;
 }
 
 // Parts a unit of four levels or more is split into, by its level-2
 // candidates.  With few units per tile the heaviest unit alone is the count's
 // time (6-cycle with chord on R-MAT 2^10, 12,016 units: 2.1 ms whole, 1.4 in
 // 6 parts).  A part forms the unit's first sets again, so units are split
-// only until there are 16 parts a tile, and not at all where a unit is one
-// level deep (house by the reference's rules on R-MAT 2^12: 1.39 ms whole,
-// 1.73 in 5 parts).
+// only until there are 16 parts a tile, light ones of sparse graphs not at all
+// (triangle prism on G(4,096, 2): 0.021 ms whole, 0.088 in parts; 6-cycle 0.069
+// and 0.089), nor where a unit is one level deep (house by the reference's
+// rules on R-MAT 2^12: 1.39 ms whole, 1.73 in 5 parts).
 constexpr int kSplitShare = 16;
 constexpr int kMostParts = 32;
 
-__host__ __device__ __forceinline__ int unit_parts(int64_t units, int64_t tiles, int basic) {
-    if (basic < 4 || units <= 0) return 1;
+__host__ __device__ __forceinline__ int unit_parts(int64_t units, int64_t tiles, int basic,
+                                                   bool light, int32_t V, int64_t E) {
+    if (basic < 4 || units <= 0 || (light && E < int64_t(kSparse) * V)) return 1;
     const int64_t p = tiles * kSplitShare / units;
     return (int)(p < 1 ? 1 : p > kMostParts ? kMostParts : p);
 }
 
-template <int G, bool STATS, bool ALL_ENTRIES = false>
-__global__ void __launch_bounds__(256, 4)
+// Plans of three levels and more, and two-level ones whose lanes cannot take
+// units alone, in three forms (kernel_form chooses):
+//  * kPlain, for graphs without bitmap rows: half as long, 64 registers, four
+//    CTAs of 256 threads an SM.  The rows' code slows a count down though it is
+//    never run (house on G(2^18, 4): 3.2 ms with it, 2.35 without);
+//  * kRows: 64 registers, four CTAs, next to no spills;
+//  * kRowsWide, for large graphs without a dense core, whose lists are short and
+//    come from L2: 40 registers, six CTAs; what it spills costs less than the
+//    latency the two more hide (Barabasi-Albert 2^20 x 2: path of five 12.4 ->
+//    10.9 ms, house 13.1 -> 11.3; but 2^18 x 8, triangle prism 5.2 -> 6.6, and
+//    R-MAT 2^18, gem 13.2 -> 14.6).
+enum Form { kPlain, kRows, kRowsWide };
+constexpr int32_t kWideVertices = 1 << 17;
+
+template <int G, bool STATS, bool ALL_ENTRIES, Form FORM>
+__global__ void __launch_bounds__(FORM == kRows ? 1024 : 256, FORM == kRowsWide ? 6 : 0)
     search_kernel(const SearchArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const Tile<G> t;
@@ -1132,25 +1166,76 @@ __global__ void __launch_bounds__(256, 4)
         a.scratch + ((int64_t)blockIdx.x * tiles_per_block + tile_in_block) *
                         a.scratch_stride;
     unsigned long long acc = 0, bytes = 0;
-    const bool pairs = !ALL_ENTRIES && P.basic == 2 && P.lane_last;
-    const int64_t tiles = (int64_t)gridDim.x * tiles_per_block;
-    int64_t left = a.num_tasks - a.task_begin;
-    // (a grab of a split queue is one part of one unit; an instrumented launch
-    // splits none: every part forms the unit's first sets again, and the bytes
-    // are the plan's, not the launch shape's)
-    const int parts = STATS ? 1 : unit_parts(left, tiles, P.basic);
+    // (the queue's shape is worked out again where it is needed: kept, it would
+    // take registers from the walk)
+    auto tiles = [&] { return (int64_t)gridDim.x * (blockDim.x / G); };
+    auto units = [&] { return a.num_tasks - a.task_begin; };
+    auto light = [&] { return light_units(P, a.cap, a.max_lower, a.V, a.off[a.V]); };
+    auto next_take = [&](int64_t left) {
+        return grab_units(left, tiles(),
+                          grab_share(units(), tiles(), light(), a.V, a.off[a.V]), 1, a.chunk);
+    };
+    if (t.lane == 0) {
+        S.first2 = 0;
+        // (a grab of a split queue is one part of one unit; an instrumented
+        // launch splits none: every part forms the unit's first sets again, and
+        // the bytes are the plan's, not the launch shape's)
+        S.step2 =
+            STATS ? 1 : unit_parts(units(), tiles(), P.basic, light(), a.V, a.off[a.V]);
+    }
+    t.sync();
+    int32_t take = next_take(units());
     for (;;) {
         unsigned long long start = 0;
+        const unsigned parts = (unsigned)S.step2;
         if (parts > 1) {
-            if (t.lane == 0) start = atomicAdd(&a.ctr->cursor, 1ull);
+            if (t.lane == 0) {
+                start = atomicAdd(&a.ctr->cursor, 1ull);
+                S.first2 = (int)(start % parts);
+            }
             start = t.bcast(start, 0);
-            const int64_t unit = a.task_begin + (int64_t)(start / (unsigned)parts);
+            const int64_t unit = a.task_begin + (int64_t)(start / parts);
             if (unit >= a.num_tasks) break;
-            run_units<G, STATS, ALL_ENTRIES>(t, S, P, a, unit, unit + 1, scratch, acc, bytes,
-                                             (int)(start % (unsigned)parts), parts);
+            t.sync();
+            run_units<G, STATS, ALL_ENTRIES, FORM != kPlain>(t, S, P, a, unit, unit + 1, scratch, acc,
+                                                   bytes);
             continue;
         }
-        const int64_t take = grab_units(left, tiles, pairs, G, a.chunk);
+        if (t.lane == 0)
+            start = (unsigned long long)a.task_begin +
+                    atomicAdd(&a.ctr->cursor, (unsigned long long)take);
+        start = t.bcast(start, 0);
+        if (start >= (unsigned long long)a.num_tasks) break;
+        const int64_t end = min((int64_t)start + take, a.num_tasks);
+        take = next_take(a.num_tasks - (int64_t)start);
+        run_units<G, STATS, ALL_ENTRIES, FORM != kPlain>(t, S, P, a, (int64_t)start, end, scratch, acc,
+                                               bytes);
+    }
+    if (t.lane == 0) {
+        atomicAdd(&a.ctr->result, acc);
+        if (STATS) atomicAdd(&a.ctr->bytes, bytes);
+    }
+}
+
+// Two-level plans whose lanes take the units one each (run_pairs).
+template <int G, bool STATS>
+__global__ void __launch_bounds__(1024)
+    pairs_kernel(const SearchArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const Tile<G> t;
+    const int tiles_per_block = blockDim.x / G;
+    const int tile_in_block = threadIdx.x / G;
+    TileSmem &S = reinterpret_cast<TileSmem *>(smem_raw)[tile_in_block];
+    const GatPlan &P = *a.plan;
+    int32_t *scratch =
+        a.scratch + ((int64_t)blockIdx.x * tiles_per_block + tile_in_block) *
+                        a.scratch_stride;
+    unsigned long long acc = 0, bytes = 0;
+    const int64_t tiles = (int64_t)gridDim.x * tiles_per_block;
+    int64_t left = a.num_tasks - a.task_begin;
+    for (;;) {
+        const int32_t take = grab_units(left, tiles, kPairShare, G, a.chunk);
+        unsigned long long start = 0;
         if (t.lane == 0)
             start = (unsigned long long)a.task_begin +
                     atomicAdd(&a.ctr->cursor, (unsigned long long)take);
@@ -1158,8 +1243,7 @@ __global__ void __launch_bounds__(256, 4)
         if (start >= (unsigned long long)a.num_tasks) break;
         left = a.num_tasks - (int64_t)start;
         const int64_t end = min((int64_t)start + take, a.num_tasks);
-        run_units<G, STATS, ALL_ENTRIES>(t, S, P, a, (int64_t)start, end, scratch, acc,
-                                         bytes);
+        run_pairs<G, STATS>(t, S, P, a, (int64_t)start, end, scratch, acc, bytes);
     }
     if (t.lane == 0) {
         atomicAdd(&a.ctr->result, acc);
@@ -1173,7 +1257,7 @@ __global__ void __launch_bounds__(256, 4)
 // running total to the job's result whenever it moves to another job, and at
 // exit.
 template <int G>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(1024)
     batch_kernel(const BatchJob *__restrict__ jobs, const int64_t *__restrict__ vstart,
                  int32_t num_jobs, int64_t vtotal, unsigned long long *cursor,
                  unsigned long long *results, int32_t *scratch_all, int64_t scratch_stride) {
@@ -1186,6 +1270,11 @@ __global__ void __launch_bounds__(256, 4)
         scratch_all + ((int64_t)blockIdx.x * tiles_per_block + tile_in_block) * scratch_stride;
     unsigned long long acc = 0, bytes = 0;
     int cur_job = -1;
+    if (t.lane == 0) {
+        S.first2 = 0;
+        S.step2 = 1;
+    }
+    t.sync();
     for (;;) {
         unsigned long long vs = 0;
         if (t.lane == 0) vs = atomicAdd(cursor, 1ull);
@@ -1200,49 +1289,56 @@ __global__ void __launch_bounds__(256, 4)
             cur_job = j;
         }
         const int64_t end = min(start + job.args.chunk, job.args.num_tasks);
-        run_units<G, false, false>(t, S, *job.args.plan, job.args, start, end, scratch, acc,
-                                   bytes);
+        const GatPlan &P = *job.args.plan;
+        if (P.basic == 2 && P.lane_last)
+            run_pairs<G, false>(t, S, P, job.args, start, end, scratch, acc, bytes);
+        else
+            run_units<G, false, false, true>(t, S, P, job.args, start, end, scratch, acc, bytes);
     }
     if (t.lane == 0 && cur_job >= 0 && acc) atomicAdd(&results[jobs[cur_job].result], acc);
 }
 
-template <int G, bool STATS>
-cudaError_t launch_one(const SearchArgs &a, int grid, int block,
-                       cudaStream_t stream) {
-    const size_t smem = size_t(block / G) * sizeof(TileSmem);
-    // Set on every launch: the attribute belongs to the current device's
-    // context, and a process may count on several devices or reset one.
-    cudaError_t e = cudaFuncSetAttribute(
-        search_kernel<G, STATS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) return e;
-    search_kernel<G, STATS><<<grid, block, smem, stream>>>(a);
-    return cudaGetLastError();
+// The kernel that walks a plan: two-level plans whose lanes take units alone
+// have one, the others three (Form).  Plans that intersect nothing have no use
+// for rows.  (Instrumented launches are kRows.)
+using SearchKernel = void (*)(SearchArgs);
+
+template <int G>
+SearchKernel kernel_form(const GatPlan &plan, const DevGraphView &g, bool rows, bool stats) {
+    if (plan.basic == 2 && plan.lane_last)
+        return stats ? pairs_kernel<G, true> : pairs_kernel<G, false>;
+    if (stats) return search_kernel<G, true, false, kRows>;
+    bool sets = false;
+    for (int p = 0; p < plan.num_prefix; p++) sets |= plan.p_kind[p] != GAT_SET_ALIAS;
+    if (!rows || !g.deep_rows || !sets) return search_kernel<G, false, false, kPlain>;
+    return g.V >= kWideVertices && g.max_lower <= kThinCore
+               ? search_kernel<G, false, false, kRowsWide>
+               : search_kernel<G, false, false, kRows>;
 }
 
-template <bool STATS>
-cudaError_t dispatch(const SearchArgs &a, int tile, int grid, int block,
-                     cudaStream_t s) {
+SearchKernel kernel_for(const GatPlan &plan, const DevGraphView &g, int tile, bool rows,
+                        bool stats) {
     switch (tile) {
-        case 1: return launch_one<1, STATS>(a, grid, block, s);
-        case 2: return launch_one<2, STATS>(a, grid, block, s);
-        case 4: return launch_one<4, STATS>(a, grid, block, s);
-        case 8: return launch_one<8, STATS>(a, grid, block, s);
-        case 16: return launch_one<16, STATS>(a, grid, block, s);
-        case 32: return launch_one<32, STATS>(a, grid, block, s);
-        default: return cudaErrorInvalidValue;
+        case 1: return kernel_form<1>(plan, g, rows, stats);
+        case 2: return kernel_form<2>(plan, g, rows, stats);
+        case 4: return kernel_form<4>(plan, g, rows, stats);
+        case 8: return kernel_form<8>(plan, g, rows, stats);
+        case 16: return kernel_form<16>(plan, g, rows, stats);
+        case 32: return kernel_form<32>(plan, g, rows, stats);
+        default: return nullptr;
     }
 }
 
-template <int G, bool STATS>
-int occupancy(int block) {
-    int n = 0;
-    const size_t smem = size_t(block / G) * sizeof(TileSmem);
-    cudaFuncSetAttribute(search_kernel<G, STATS>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &n, search_kernel<G, STATS>, block, smem) != cudaSuccess)
-        return 0;
-    return n;
+// Set on every launch: the attribute belongs to the current device's context,
+// and a process may count on several devices or reset one.
+cudaError_t allow_smem(SearchKernel k) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+}
+
+size_t block_smem(int block, int tile) { return size_t(block / tile) * sizeof(TileSmem); }
+
+bool has_rows(const DevGraphView &g, const LaunchShape &shape) {
+    return shape.use_bitmaps && g.bitmaps != nullptr && g.hub_slot != nullptr;
 }
 
 // One CTA per hub (grid-stride over hubs): sets bit x of the hub's row for
@@ -1291,7 +1387,10 @@ void batch_fill_job(void *dst, const GatPlan *d_plan, const GatPlan &h_plan,
     a.task_begin = num_shards > 0 ? total * shard / num_shards : 0;
     a.num_tasks = num_shards > 0 ? total * (shard + 1) / num_shards : total;
     a.linear_below = linear_below;
-    const bool hubs = use_bitmaps && g.bitmaps != nullptr && g.hub_slot != nullptr;
+    a.max_lower = g.max_lower;
+    const bool pairs = h_plan.basic == 2 && h_plan.lane_last;
+    const bool hubs = use_bitmaps && g.bitmaps != nullptr && g.hub_slot != nullptr &&
+                      (pairs || g.deep_rows);
     a.hub_slot = hubs ? g.hub_slot : nullptr;
     a.bitmaps = hubs ? g.bitmaps : nullptr;
     a.bitmap_words = hubs ? g.bitmap_words : 0;
@@ -1303,11 +1402,17 @@ int64_t batch_job_tasks(const void *job) {
     return a.num_tasks - a.task_begin;
 }
 
-int64_t batch_job_grabs(void *job, const GatPlan &plan, int64_t tiles, int tile, int chunk) {
+int64_t batch_job_grabs(void *job, const GatPlan &plan, int64_t E, int64_t tiles, int tile,
+                        int chunk) {
     SearchArgs &a = reinterpret_cast<BatchJob *>(job)->args;
     const bool pairs = plan.basic == 2 && plan.lane_last;
     const int64_t n = a.num_tasks - a.task_begin;
-    a.chunk = (int32_t)grab_units(n, tiles, pairs, tile, int64_t(chunk) * (pairs ? tile : 1));
+    const int share =
+        pairs ? kPairShare
+              : grab_share(n, tiles, light_units(plan, a.cap, a.max_lower, a.V, E), a.V, E);
+    const int unit = pairs ? tile : 1;
+    a.chunk = grab_units(n, tiles, share, unit,
+                         (int32_t)std::min<int64_t>(int64_t(chunk) * unit, 1 << 24));
     return (n + a.chunk - 1) / a.chunk;
 }
 
@@ -1369,19 +1474,15 @@ cudaError_t launch_batch(const void *d_jobs, const int64_t *d_vstart, int32_t nu
 #undef GAT_BL
 }
 
-int blocks_per_sm(int tile, int block, bool stats) {
-#define GAT_OCC(G) \
-    return stats ? occupancy<G, true>(block) : occupancy<G, false>(block)
-    switch (tile) {
-        case 1: GAT_OCC(1);
-        case 2: GAT_OCC(2);
-        case 4: GAT_OCC(4);
-        case 8: GAT_OCC(8);
-        case 16: GAT_OCC(16);
-        case 32: GAT_OCC(32);
-        default: return 0;
-    }
-#undef GAT_OCC
+int blocks_per_sm(const GatPlan &plan, const DevGraphView &g, const LaunchShape &shape,
+                  bool stats) {
+    const SearchKernel k = kernel_for(plan, g, shape.tile, has_rows(g, shape), stats);
+    int n = 0;
+    if (!k || allow_smem(k) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &n, k, shape.block, block_smem(shape.block, shape.tile)) != cudaSuccess)
+        return 0;
+    return n;
 }
 
 int64_t tile_scratch_ints(const GatPlan &plan, int32_t max_degree) {
@@ -1410,12 +1511,16 @@ cudaError_t launch_search(const GatPlan *d_plan, const GatPlan &h_plan,
     a.scratch_stride = scratch_stride;
     a.chunk = shape.chunk > 0 ? shape.chunk : 1;
     a.linear_below = shape.linear_below;
-    const bool hubs = shape.use_bitmaps && g.bitmaps != nullptr && g.hub_slot != nullptr;
+    a.max_lower = g.max_lower;
+    const bool hubs = has_rows(g, shape);
     a.hub_slot = hubs ? g.hub_slot : nullptr;
     a.bitmaps = hubs ? g.bitmaps : nullptr;
     a.bitmap_words = hubs ? g.bitmap_words : 0;
-    return stats ? dispatch<true>(a, shape.tile, shape.grid, shape.block, stream)
-                 : dispatch<false>(a, shape.tile, shape.grid, shape.block, stream);
+    const SearchKernel k = kernel_for(h_plan, g, shape.tile, hubs, stats);
+    if (!k) return cudaErrorInvalidValue;
+    if ((e = allow_smem(k)) != cudaSuccess) return e;
+    k<<<shape.grid, shape.block, block_smem(shape.block, shape.tile), stream>>>(a);
+    return cudaGetLastError();
 }
 
 }  // namespace gat
@@ -1463,18 +1568,18 @@ template <int G>
 cudaError_t noalloc_launch(const SearchArgs &a, int block, int max_grid, int sms,
                            cudaStream_t stream) {
     const size_t smem = size_t(block / G) * sizeof(TileSmem);
-    cudaError_t e = cudaFuncSetAttribute(search_kernel<G, false, true>,
+    cudaError_t e = cudaFuncSetAttribute(search_kernel<G, false, true, kPlain>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          227 * 1024);
     if (e != cudaSuccess) return e;
     int occ = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, search_kernel<G, false, true>,
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, search_kernel<G, false, true, kPlain>,
                                                       block, smem);
     if (e != cudaSuccess) return e;
     if (occ < 1) return cudaErrorInvalidConfiguration;
     int grid = sms * occ;
     if (max_grid > 0 && grid > max_grid) grid = max_grid;
-    search_kernel<G, false, true><<<grid, block, smem, stream>>>(a);
+    search_kernel<G, false, true, kPlain><<<grid, block, smem, stream>>>(a);
     return cudaGetLastError();
 }
 
@@ -1541,6 +1646,7 @@ int count_noalloc(const GatPlan &plan, const int64_t *d_off, const int32_t *d_ad
     a.scratch_stride = stride;
     a.chunk = shape.chunk > 0 ? shape.chunk : 1;
     a.linear_below = shape.linear_below;
+    a.max_lower = INT32_MAX;  // not known
     a.hub_slot = nullptr;
     a.bitmaps = nullptr;
     a.bitmap_words = 0;

@@ -26,6 +26,7 @@ struct DevGraphView {
     const int32_t *hub_slot = nullptr;
     const uint32_t *bitmaps = nullptr;
     int64_t bitmap_words = 0;  // words per row: ceil(V / 32), up to whole 16-byte groups
+    bool deep_rows = false;    // worth their while to plans of three levels and more
 };
 
 // Fills one V-bit row per hub (rows must be zeroed first).
@@ -49,7 +50,8 @@ struct CsrExtremes {
 cudaError_t csr_extremes_device(const int64_t *off, const int64_t *lo_off, int32_t V,
                                 int64_t light_below, bool ordered, CsrExtremes *out,
                                 cudaStream_t stream);
-// On a degree-ordered copy: out[0] rows of degree >= d0, out[1] of >= d1.
+// On a degree-ordered copy: for d0 and d1 in turn the rows of at least that
+// degree and the entries they hold (out[0 .. 3]).
 cudaError_t leading_rows_device(const int64_t *off, int32_t V, int64_t d0, int64_t d1,
                                 int64_t *out, cudaStream_t stream);
 // slot[v] = bitmap row of v or -1.  ordered: rows 0 .. n-1 are the vertices
@@ -192,7 +194,8 @@ void batch_fill_job(void *dst, const GatPlan *d_plan, const GatPlan &h_plan,
 int64_t batch_job_tasks(const void *job);
 // Fixes the job's units per grab (at most `chunk`, per lane for two-level
 // plans) on `tiles` resident tiles; returns the job's grabs.
-int64_t batch_job_grabs(void *job, const GatPlan &plan, int64_t tiles, int tile, int chunk);
+int64_t batch_job_grabs(void *job, const GatPlan &plan, int64_t E, int64_t tiles, int tile,
+                        int chunk);
 int batch_blocks_per_sm(int tile, int block);
 cudaError_t launch_batch(const void *d_jobs, const int64_t *d_vstart, int32_t num_jobs,
                          int64_t vtotal, int tile, int grid, int block,
@@ -216,8 +219,10 @@ enum : unsigned long long {
 
 // Shared memory one tile needs.
 size_t tile_smem_bytes();
-// Largest CTA count per SM for this tile/block/stats combination.
-int blocks_per_sm(int tile, int block, bool stats);
+// Largest CTA count per SM of the kernel that launch_search takes for these
+// (0: the shape is not one).  `plan` is the plan as the device will see it.
+int blocks_per_sm(const GatPlan &plan, const DevGraphView &g, const LaunchShape &shape,
+                  bool stats);
 // Scratch ints one tile needs for `plan` on a graph with this max degree.
 int64_t tile_scratch_ints(const GatPlan &plan, int32_t max_degree);
 

@@ -116,7 +116,8 @@ __global__ void leading_rows_kernel(const int64_t *__restrict__ off, int32_t V, 
         lo = right ? v + 1 : lo;
         n = right ? n - h - 1 : h;
     }
-    out[threadIdx.x] = lo;
+    out[2 * threadIdx.x] = lo;
+    out[2 * threadIdx.x + 1] = off[lo];
 }
 
 // The bounds of the 4-cycle kernels' counter widths, likewise.

@@ -10,7 +10,7 @@ CSRC = ROOT / "graphautotune_b200" / "csrc"
 SOURCES = [HERE / "fake_gpu.cpp", *(CSRC / f"{n}.cpp" for n in
                                     ("schedule", "plan", "graph", "devmem", "capi"))]
 SLOTS = ("refuse", "throw", "misuse", "live", "pending", "c5_launches", "c5_grid", "c5_bitmaps",
-         "searches", "cliques")
+         "searches", "cliques", "deep_rows")
 NEVER = 2 ** 63 - 1
 
 

@@ -29,6 +29,7 @@ enum {
     kC5Bitmaps,   // 1: the last 5-cycle launch was given bitmaps
     kSearches,
     kCliques,
+    kDeepRows,    // the last search's DevGraphView::deep_rows
     kSlots
 };
 extern "C" {
@@ -275,10 +276,11 @@ cudaError_t csr_extremes_device(const int64_t *off, const int64_t *lo_off, int32
 
 cudaError_t leading_rows_device(const int64_t *off, int32_t V, int64_t d0, int64_t d1,
                                 int64_t *out, cudaStream_t) {
-    out[0] = out[1] = 0;
-    for (int32_t v = 0; v < V; v++) {
-        out[0] += off[v + 1] - off[v] >= d0;
-        out[1] += off[v + 1] - off[v] >= d1;
+    const int64_t want[2] = {d0, d1};
+    for (int i = 0; i < 2; i++) {
+        out[2 * i] = 0;
+        for (int32_t v = 0; v < V; v++) out[2 * i] += off[v + 1] - off[v] >= want[i];
+        out[2 * i + 1] = off[out[2 * i]];
     }
     return cudaSuccess;
 }
@@ -316,7 +318,7 @@ cudaError_t pairs_csr_device(const int32_t *, int64_t, int32_t, int64_t *, int32
 
 // --------------------------------------------------------- kernels that count
 
-int blocks_per_sm(int, int, bool) { return 4; }
+int blocks_per_sm(const GatPlan &, const DevGraphView &, const LaunchShape &, bool) { return 4; }
 int batch_blocks_per_sm(int, int) { return 4; }
 int64_t tile_scratch_ints(const GatPlan &plan, int32_t max_degree) {
     return int64_t(plan.num_store) * max_degree;
@@ -326,6 +328,7 @@ cudaError_t launch_search(const GatPlan *, const GatPlan &, const DevGraphView &
                           cudaStream_t) {
     check(g, shape.use_bitmaps && g.bitmaps && g.hub_slot);
     fake_state[kSearches]++;
+    fake_state[kDeepRows] = g.deep_rows;
     return *ctr = DevCounters{}, cudaSuccess;
 }
 int count_noalloc(const GatPlan &, const int64_t *, const int32_t *, int32_t, int64_t, int32_t,
@@ -370,7 +373,7 @@ void batch_fill_job(void *dst, const GatPlan *, const GatPlan &, const DevGraphV
     *static_cast<FakeJob *>(dst) = {g, bitmaps && g.bitmaps && g.hub_slot, result};
 }
 int64_t batch_job_tasks(const void *job) { return static_cast<const FakeJob *>(job)->g.lo_total; }
-int64_t batch_job_grabs(void *job, const GatPlan &, int64_t, int, int) { return batch_job_tasks(job); }
+int64_t batch_job_grabs(void *job, const GatPlan &, int64_t, int64_t, int, int) { return batch_job_tasks(job); }
 cudaError_t launch_batch(const void *jobs, const int64_t *, int32_t n, int64_t, int, int, int,
                          unsigned long long *, unsigned long long *, int32_t *, int64_t,
                          cudaStream_t) {
