@@ -30,15 +30,16 @@
 //    next window.  Once the wedges left fit the CTA table, the lists'
 //    remainders go through the table in one pass.
 //
-// Bound: on chip.  DRAM is at 1% and L2 at 12% of their peaks; a shared
-// atomic of 32 random counters takes 4.4 wavefronts, and a root's barriers
-// and chains of dependent reads cost more than its counting for all but the
-// largest thousand.  R-MAT 2^20 (5.65e9 wedges) on a B200, ms per CTA: roots
-// of a million wedges and more 5.1 (76% of all wedges), others 3.3, reading
-// counters out 2, finding segments 1.3, tables 1.5; the light kernel 0.9.
-// One count: 21.4 ms with a search per entry, 16-bit windows and a lane per
-// list in the light kernel, now 12.6; R-MAT 2^18 3.2 -> 2.15, Barabasi-Albert
-// 60,000 x 9 0.66 -> 0.23.
+// Bound: on chip.  On R-MAT 2^18 DRAM is at 0.2% and L2 at 8% of their peaks
+// and issue slots are 55% busy; barriers and list loads stall a warp about
+// equally (3.3 and 3.1 per instruction).  A shared atomic of 32 random counters
+// takes 4.4 wavefronts, and a root's barriers and chains of dependent reads cost
+// more than its counting for all but the largest thousand.  R-MAT 2^20 (5.65e9
+// wedges) on a B200, ms per CTA: roots of a million wedges and more 5.1 (76% of
+// all wedges), others 3.3, reading counters out 2, finding segments 1.3, tables
+// 1.5; the light kernel 0.25.  One count: 21.4 ms with a search per entry, 16-bit
+// windows and a lane per list in the light kernel, now 12.1; R-MAT 2^18 3.2 ->
+// 2.04, Barabasi-Albert 60,000 x 9 0.66 -> 0.23.
 //
 // Neither kernel waits on another CTA; the deferred list is written by the
 // first launch and read by the second, ordered on the stream.
